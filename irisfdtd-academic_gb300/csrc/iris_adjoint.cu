@@ -456,6 +456,7 @@ template <typename T> int adj_forward(iris_adjoint* J, int nsteps) {
   CK(cudaMemsetAsync(F->fd, 0, (size_t)F->P * F->p.nof * 16, F->st));
   F->fd_zero = false;
   F->nslot = 0;
+  F->tf_end = 0;
   CK(cudaEventRecord(J->ev[0], F->st));
   for (int it = 1; it <= nsteps; ++it) {
     const int seg = (it - 1) / J->K;
@@ -464,7 +465,7 @@ template <typename T> int adj_forward(iris_adjoint* J, int nsteps) {
       if (rc) return rc;
     }
     if (seg == S - 1) adj_record<T>(J, it - 1 - seg * J->K);
-    one_step(F, it, true);
+    one_step(F, it, nsteps + 1 - it, true);
   }
   dft_flush(F);
   CK(cudaEventRecord(J->ev[1], F->st));
@@ -494,9 +495,10 @@ template <typename T> int adj_backward(iris_adjoint* J) {
       CK(cudaEventRecord(J->ev[0], F->st));
       rc = ckpt_io(J, seg, false);
       if (rc) return rc;
+      F->tf_end = 0;
       for (int it = s0; it <= s1; ++it) {
         adj_record<T>(J, it - s0);
-        one_step(F, it, false);
+        one_step(F, it, s1 + 1 - it, false);
       }
       CK(cudaEventRecord(J->ev[1], F->st));
       CK(cudaEventSynchronize(J->ev[1]));

@@ -41,7 +41,7 @@ struct BItem {
   int cell, x0, y0, z0;  // tile origin (1-based)
 };
 struct TItem {
-  int cell, ix0, iy0, pad;
+  int cell, ix0, iy0, col;  // col: table column of ix0
 };
 struct BSeg {
   Seg s;
@@ -60,6 +60,7 @@ constexpr int NTILES = 8, FLAT = 5, FUSED = 7;
 constexpr int TILES[NTILES][3] = {{32, 8, 1}, {32, 4, 2}, {64, 4, 1}, {16, 16, 1},
                                   {32, 2, 4}, {256, 1, 1}, {256, 1, 1}, {FZ_X, FZ_Y, 1}};
 constexpr int FB_CHUNK = 64;  // planes per FUSED item outside the UPML slabs
+constexpr int TFSF_YCH = 16;  // rows of a TF/SF item
 static_assert(NTILES == IRIS_BATCH_NTILES, "the ABI's candidate count");
 
 // Copies the cell's arguments into shared memory when the item's cell changes.
@@ -174,18 +175,35 @@ __global__ void __launch_bounds__(FZ_X* FZ_Y, 2) k_batch_fused(const FusedArgs* 
   }
 }
 
+// The TF/SF corrections of steps it0 .. it0+n-1 (from *itp on when given) for
+// every column of every cell: column q of a table row is column cols[q].y of
+// cell cols[q].x.
 template <typename T>
-__global__ void __launch_bounds__(64) k_batch_tfsf(const FieldArgs<T>* __restrict__ args,
-                                                   const SrcArgs* __restrict__ srcs, const TItem* __restrict__ items,
-                                                   long nitems, int it, const int* itp) {
-  if (itp) it += *itp;
+__global__ void __launch_bounds__(128) k_batch_tfsf_table(const SrcArgs* __restrict__ srcs, const int2* __restrict__ cols,
+                                                          int it0, const int* itp, int n, int ncol,
+                                                          TfsfVal<T>* __restrict__ out) {
+  const long j = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= (long)n * ncol) return;
+  if (itp) it0 += *itp;
+  const int2 c = cols[j % ncol];
+  out[j] = tfsf_entry<T>(srcs[c.x], it0 + (int)(j / ncol), c.y);
+}
+
+// One step's corrections of every cell from its table row: items of 64
+// columns by TFSF_YCH rows.
+template <typename T>
+__global__ void __launch_bounds__(256) k_batch_tfsf(const FieldArgs<T>* __restrict__ args,
+                                                    const SrcArgs* __restrict__ srcs, const TItem* __restrict__ items,
+                                                    long nitems, const TfsfVal<T>* __restrict__ row) {
   for (long k = blockIdx.x; k < nitems; k += gridDim.x) {
     const TItem b = items[k];
     const FieldArgs<T>& a = args[b.cell];
     const SrcArgs& s = srcs[b.cell];
     const int ix = b.ix0 + threadIdx.x;
-    if (s.variant == 0 || ix > s.nx + 1) continue;
-    tfsf_column<T>(a.e, a.h, a.g, s, it, ix, b.iy0, min(b.iy0 + TFSF_YCH - 1, s.ny + 1));
+    if (ix > s.nx + 1) continue;
+    const TfsfVal<T> t = row[b.col + threadIdx.x];
+    for (int iy = b.iy0 + threadIdx.y; iy <= min(b.iy0 + TFSF_YCH - 1, s.ny + 1); iy += 4)
+      tfsf_apply<T>(a.e, a.h, a.g, s, ix, iy, t);
   }
 }
 
@@ -228,6 +246,11 @@ struct iris_batch {
   int grid_e = 0, grid_h = 0;
   TItem* d_titems = nullptr;
   long ntitems = 0;
+  // TF/SF table of all cells' columns, tfcap steps: those of [tf_at, tf_end)
+  // within a call
+  int2* d_tcols = nullptr;
+  void* d_tfv = nullptr;
+  int ntcols = 0, tfcap = 0, tf_at = 0, tf_end = 0;
   BSeg* d_bsegs = nullptr;
   int nbsegs = 0;
   long max_seg = 0;
@@ -506,8 +529,9 @@ template <typename T> void batch_eh(iris_batch* B, bool e) {
 }
 
 // One step of every cell: step it, or *itp + it when itp is given; sampled
-// says whether the step's DFT sample is taken.
-template <typename T> void batch_one_step(iris_batch* B, int it, const int* itp, bool sampled) {
+// says whether the step's DFT sample is taken, left the steps to take, it
+// included.
+template <typename T> void batch_one_step(iris_batch* B, int it, int left, const int* itp, bool sampled) {
   iris_engine* M = B->master;
   const iris_params& p = M->p;
   using V = typename V2<T>::t;
@@ -520,8 +544,16 @@ template <typename T> void batch_one_step(iris_batch* B, int it, const int* itp,
   const FieldArgs<T>* args = cur_args<T>(B);  // after the fused pass: the new set
   if (B->ntitems) {
     KTimer tm(M, IRIS_KC_TFSF);
-    const long g = std::min<long>(B->ntitems, 152L * 16);
-    k_batch_tfsf<T><<<(unsigned)g, 64, 0, M->st>>>(args, B->d_src, B->d_titems, B->ntitems, it, itp);
+    if (it < B->tf_at || it >= B->tf_end) {
+      const int n = std::max(1, std::min(left, B->tfcap));
+      k_batch_tfsf_table<T><<<(unsigned)(((long)n * B->ntcols + 127) / 128), 128, 0, M->st>>>(
+          B->d_src, B->d_tcols, it, itp, n, B->ntcols, (TfsfVal<T>*)B->d_tfv);
+      B->tf_at = it;
+      B->tf_end = it + n;
+    }
+    const long g = std::min<long>(B->ntitems, 152L * 8);
+    k_batch_tfsf<T><<<(unsigned)g, dim3(64, 4), 0, M->st>>>(args, B->d_src, B->d_titems, B->ntitems,
+                                                            (const TfsfVal<T>*)B->d_tfv + (long)(it - B->tf_at) * B->ntcols);
   }
   if (sampled) {
     {
@@ -538,17 +570,20 @@ template <typename T> void batch_one_step(iris_batch* B, int it, const int* itp,
 template <typename T> int batch_step_t(iris_batch* B, int it0, int n) {
   iris_engine* M = B->master;
   const iris_params& p = M->p;
+  B->tf_end = 0;
   int it = it0;
   while (it < it0 + n) {
     if (graph_ready(M, it, it0 + n - it)) {
       int rc = graph_block(M, it, [&] {
-        for (int j = 0; j < M->K; ++j) batch_one_step<T>(B, j, M->d_it, true);
+        B->tf_end = 0;
+        for (int j = 0; j < M->K; ++j) batch_one_step<T>(B, j, M->K - j, M->d_it, true);
       });
+      B->tf_end = 0;
       if (rc) return rc;
       it += M->K;
       continue;
     }
-    batch_one_step<T>(B, it, nullptr, M->P > 0 && it >= p.to_fourier && it % p.sample_fourier == 0);
+    batch_one_step<T>(B, it, it0 + n - it, nullptr, M->P > 0 && it >= p.to_fourier && it % p.sample_fourier == 0);
     ++it;
   }
   B->steps_taken += n;
@@ -559,7 +594,8 @@ template <typename T> int batch_step_t(iris_batch* B, int it0, int n) {
 void batch_free(iris_batch* B) {
   for (iris_engine* E : B->cells)
     if (E) iris_destroy(E);
-  void* ptrs[] = {B->d_args, B->d_src, B->d_items, B->d_titems, B->d_bsegs, B->d_fargs, B->d_fitems};
+  void* ptrs[] = {B->d_args, B->d_src, B->d_items, B->d_titems, B->d_bsegs, B->d_fargs, B->d_fitems,
+                  B->d_tcols, B->d_tfv};
   for (void* q : ptrs)
     if (q) cudaFree(q);
   if (B->master) {
@@ -600,6 +636,7 @@ int iris_batch_create(int ncells, const iris_params* params, const double* fw, i
   std::vector<FluxFace> faces(6 * (size_t)ncells);
   std::vector<SrcArgs> srcs(ncells);
   std::vector<TItem> titems;
+  std::vector<int2> tcols;
   for (int c = 0; c < ncells; ++c) {
     iris_params q = params[c];
     q.stencil = IRIS_STENCIL_SPLIT;
@@ -626,9 +663,12 @@ int iris_batch_create(int ncells, const iris_params* params, const double* fw, i
       faces[6 * c + f] = ff;
     }
     srcs[c] = E->src;
-    if (E->src.variant != 0)
+    if (E->src.variant != 0) {
+      const int col = (int)tcols.size();
       for (int iy = 0; iy <= q.ny + 1; iy += TFSF_YCH)
-        for (int ix = 0; ix <= q.nx + 1; ix += 64) titems.push_back(TItem{c, ix, iy, 0});
+        for (int ix = 0; ix <= q.nx + 1; ix += 64) titems.push_back(TItem{c, ix, iy, col + ix});
+      for (int ix = 0; ix <= q.nx + 1; ++ix) tcols.push_back(make_int2(c, ix));
+    }
     P += E->P;
   }
   // the shell: one stream, the timers and the shared DFT buffers
@@ -645,13 +685,19 @@ int iris_batch_create(int ncells, const iris_params* params, const double* fw, i
     return bail(fail(IRIS_ECUDA, "cudaStreamCreate failed"));
   int rc = alloc_dft(M, faces.data(), (int)faces.size());
   if (rc) return bail(rc);
+  // at most 1024 steps and 8 MB
+  B->ntcols = (int)tcols.size();
+  B->tfcap = (int)std::max(1L, std::min(1024L, (8L << 20) / (32L * std::max(1, B->ntcols))));
   if (cudaMalloc(&B->d_bsegs, sizeof(BSeg) * std::max<size_t>(1, bsegs.size())) != cudaSuccess ||
       cudaMalloc(&B->d_src, sizeof(SrcArgs) * ncells) != cudaSuccess ||
-      cudaMalloc(&B->d_titems, sizeof(TItem) * std::max<size_t>(1, titems.size())) != cudaSuccess)
+      cudaMalloc(&B->d_titems, sizeof(TItem) * std::max<size_t>(1, titems.size())) != cudaSuccess ||
+      cudaMalloc(&B->d_tcols, sizeof(int2) * std::max<size_t>(1, tcols.size())) != cudaSuccess ||
+      cudaMalloc(&B->d_tfv, sizeof(TfsfVal<double>) * std::max<size_t>(1, tcols.size()) * B->tfcap) != cudaSuccess)
     return bail(fail(IRIS_ENOMEM, "batch tables: allocation failed"));
   cudaMemcpy(B->d_bsegs, bsegs.data(), sizeof(BSeg) * bsegs.size(), cudaMemcpyHostToDevice);
   cudaMemcpy(B->d_src, srcs.data(), sizeof(SrcArgs) * ncells, cudaMemcpyHostToDevice);
   cudaMemcpy(B->d_titems, titems.data(), sizeof(TItem) * titems.size(), cudaMemcpyHostToDevice);
+  cudaMemcpy(B->d_tcols, tcols.data(), sizeof(int2) * tcols.size(), cudaMemcpyHostToDevice);
   B->nbsegs = (int)bsegs.size();
   B->ntitems = (long)titems.size();
   rc = batch_upload_args(B);

@@ -357,8 +357,7 @@ __device__ __forceinline__ void h_split_cell(const FieldArgs<T>& a, int x, int y
 // (code/tfsf.f90:359-517) evaluated in FP64 at the two planes the update
 // reads, then tfsf_update_3DArray (code/tfsf.f90:76-153) or
 // tfsf_update_2DArray (code/tfsf.f90:163-227) over the reference's ranges,
-// ghosts included.  The incident field is y-independent, so each thread
-// evaluates it once for its ix and walks a chunk of iy.
+// ghosts included.  The incident field is y-independent.
 
 struct SrcArgs {
   int variant;  // 0 none, 1 update_3DArray, 2 update_2DArray
@@ -443,27 +442,42 @@ __device__ inline void incident(const SrcArgs& s, int ix, int iz, int it, cx<dou
   }
 }
 
-// Add (sgn=+1) or subtract an FP64 correction to a stored field value.
-template <typename T> __device__ __forceinline__ void corr(typename V2<T>::t* p, cx<double> v, int sgn);
-template <> __device__ __forceinline__ void corr<double>(double2* p, cx<double> v, int sgn) {
-  double2 a = *p;
-  if (sgn > 0) { a.x = da(a.x, v.re); a.y = da(a.y, v.im); }
-  else { a.x = ds(a.x, v.re); a.y = ds(a.y, v.im); }
-  *p = a;
+// An FP64 correction as the field update adds it: itself in FP64; in FP32 a
+// pair of floats, its leading part and the rest (48 bits).  On GB300 an FP64
+// add of a float (two conversions and the add for each part, two a cycle per
+// SM) made the corrected planes the slowest of a step; the pair's sum costs
+// seven FP32 adds.
+template <typename T> struct TfNum;
+template <> struct TfNum<double> { using t = double; };
+template <> struct TfNum<float> { using t = float2; };
+template <typename T> __device__ __forceinline__ typename TfNum<T>::t tf_num(double v);
+template <> __device__ __forceinline__ double tf_num<double>(double v) { return v; }
+template <> __device__ __forceinline__ float2 tf_num<float>(double v) {
+  const float hi = (float)v;
+  return make_float2(hi, (float)(v - (double)hi));
 }
-template <> __device__ __forceinline__ void corr<float>(float2* p, cx<double> v, int sgn) {
-  float2 a = *p;
-  if (sgn > 0) { a.x = (float)((double)a.x + v.re); a.y = (float)((double)a.y + v.im); }
-  else { a.x = (float)((double)a.x - v.re); a.y = (float)((double)a.y - v.im); }
-  *p = a;
+// a + v (sgn > 0) or a - v, rounded once: in FP32 TwoSum of a and the leading
+// part, then the sum's error and the rest together.  A sum that is not finite
+// is returned as it is.
+__device__ __forceinline__ double tf_add(double a, double v, int sgn) { return sgn > 0 ? da(a, v) : ds(a, v); }
+__device__ __forceinline__ float tf_add(float a, float2 v, int sgn) {
+  const float h = sgn > 0 ? v.x : -v.x, l = sgn > 0 ? v.y : -v.y;
+  const float s = __fadd_rn(a, h), b = __fsub_rn(s, a);
+  const float e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, b)), __fsub_rn(h, b));
+  const float r = __fadd_rn(s, __fadd_rn(e, l));
+  return fabsf(s) <= 3.402823466e38f ? r : s;
+}
+template <typename T>
+__device__ __forceinline__ cx<T> tf_add(cx<T> a, typename TfNum<T>::t re, typename TfNum<T>::t im, int sgn) {
+  return {tf_add(a.re, re, sgn), tf_add(a.im, im, sgn)};
 }
 
-constexpr int TFSF_YCH = 16;
-
-// The two corrections of one column at one step, as tabulated for the
-// persistent kernel.
-struct __align__(32) TfsfVal {
-  double er, ei, hr, hi;  // vE, vH
+// The two corrections of one column at one step, as tabulated for a span of
+// steps: the incident field (exp, sincos and divisions in FP64, a dependent
+// chain of a few hundred FP64 instructions) is evaluated for many steps and
+// columns at once instead of in front of every step.
+template <typename T> struct __align__(32) TfsfVal {
+  typename TfNum<T>::t er, ei, hr, hi;
 };
 
 // The two corrections of column ix at step it: vE (added to or subtracted
@@ -488,47 +502,44 @@ __device__ __forceinline__ void tfsf_values(const SrcArgs& s, int it, int ix, cx
   }
 }
 
-// The corrections of column ix over the rows iy in [y0, y1]
-// (code/tfsf.f90:76-153, :163-227).
+template <typename T> __device__ __forceinline__ TfsfVal<T> tfsf_entry(const SrcArgs& s, int it, int ix) {
+  cx<double> vE, vH;
+  tfsf_values(s, it, ix, vE, vH);
+  return {tf_num<T>(vE.re), tf_num<T>(vE.im), tf_num<T>(vH.re), tf_num<T>(vH.im)};
+}
+
+// The corrections t of column ix at row iy (code/tfsf.f90:76-153, :163-227).
 template <typename T>
 __device__ __forceinline__ void tfsf_apply(typename V2<T>::t* e, typename V2<T>::t* h, const Geo& g,
-                                           const SrcArgs& s, int ix, int y0, int y1, cx<double> vE, cx<double> vH) {
+                                           const SrcArgs& s, int ix, int iy, const TfsfVal<T>& t) {
   const int zm = s.iz_min;
-  if (!bc_ok(ix >= 0 && ix <= s.nx + 1 && y0 >= 0 && y1 <= s.ny + 1 && zm >= 1 && zm <= g.nz, BC_TFSF,
-             ((long)ix << 32) | (unsigned)y1))
+  if (!bc_ok(ix >= 0 && ix <= s.nx + 1 && iy >= 0 && iy <= s.ny + 1 && zm >= 1 && zm <= g.nz, BC_TFSF,
+             ((long)ix << 32) | (unsigned)iy))
     return;
+  auto corr = [&](typename V2<T>::t* p, typename TfNum<T>::t re, typename TfNum<T>::t im, int sgn) {
+    st<T>(p, tf_add<T>(ld<T>(p), re, im, sgn));
+  };
   if (s.variant == 1) {
     if (s.i_pol == 2) {
       // E_x(iz_min) += eps_in(1)*tf5(iz_min-1): ix in [0,nx], iy in [0,ny+1]
       // H_y(iz_min-1) += dtcq2*tf1(iz_min):      ix in [0,nx], iy in [0,ny+1]
-      for (int iy = y0; iy <= y1; ++iy) {
-        if (ix <= s.nx && iy <= s.ny + 1) corr<T>(e + g.at(ix, iy, zm), vE, +1);
-        if (ix <= s.nx && iy <= s.ny + 1) corr<T>(h + g.comp + g.at(ix, iy, zm - 1), vH, +1);
+      if (ix <= s.nx) {
+        corr(e + g.at(ix, iy, zm), t.er, t.ei, +1);
+        corr(h + g.comp + g.at(ix, iy, zm - 1), t.hr, t.hi, +1);
       }
     } else {
       // E_y(iz_min) -= eps_in(1)*tf4(iz_min-1): ix in [0,nx+1], iy in [0,ny]
       // H_x(iz_min-1) -= dtcq2*tf2(iz_min):      ix in [0,nx+1], iy in [0,ny]
-      for (int iy = y0; iy <= y1; ++iy) {
-        if (ix <= s.nx + 1 && iy <= s.ny) corr<T>(e + g.comp + g.at(ix, iy, zm), vE, -1);
-        if (ix <= s.nx + 1 && iy <= s.ny) corr<T>(h + g.at(ix, iy, zm - 1), vH, -1);
+      if (iy <= s.ny) {
+        corr(e + g.comp + g.at(ix, iy, zm), t.er, t.ei, -1);
+        corr(h + g.at(ix, iy, zm - 1), t.hr, t.hi, -1);
       }
     }
   } else if (s.variant == 2) {
     // E_x(iz_min) += tf5(iz_min)/eps ; H_y(iz_min) += dtcq2*tf1(iz_min)
-    for (int iy = y0; iy <= y1; ++iy) {
-      corr<T>(e + g.at(ix, iy, zm), vE, +1);
-      corr<T>(h + g.comp + g.at(ix, iy, zm), vH, +1);
-    }
+    corr(e + g.at(ix, iy, zm), t.er, t.ei, +1);
+    corr(h + g.comp + g.at(ix, iy, zm), t.hr, t.hi, +1);
   }
-}
-
-// Incident field at ix and the corrections of the rows iy in [y0, y1].
-template <typename T>
-__device__ __forceinline__ void tfsf_column(typename V2<T>::t* e, typename V2<T>::t* h, const Geo& g,
-                                            const SrcArgs& s, int it, int ix, int y0, int y1) {
-  cx<double> vE, vH;
-  tfsf_values(s, it, ix, vE, vH);
-  tfsf_apply<T>(e, h, g, s, ix, y0, y1, vE, vH);
 }
 
 // ---------------------------------------------------------------------------

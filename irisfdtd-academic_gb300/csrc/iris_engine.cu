@@ -388,18 +388,26 @@ __global__ void __launch_bounds__(SX* SY) k_stream_h(FieldArgs<float> a, int* er
   stream_tile_h(a, 1 + blockIdx.x * SX, 1 + blockIdx.y * SY, 1 + blockIdx.z * SZC, (StageH*)smem, bar, par, err);
 }
 
+// The TF/SF corrections of steps it0 .. it0+n-1 for every column ix in
+// [0, nx+1]; the steps count from *itp when itp is given (a device-resident
+// step base, which lets a captured graph of steps be replayed at any step).
 template <typename T>
-// The step is it, or *itp + it when itp is given (a device-resident step
-// base, which lets a captured graph of steps be replayed at any step).
-__global__ void __launch_bounds__(64) k_tfsf(typename V2<T>::t* e, typename V2<T>::t* h, Geo g, SrcArgs s, int it,
-                                             const int* itp) {
-  const int ix = blockIdx.x * blockDim.x + threadIdx.x;
-  if (ix > s.nx + 1) return;
-  if (itp) it += *itp;
-  const int y0 = blockIdx.y * TFSF_YCH;
-  tfsf_column<T>(e, h, g, s, it, ix, y0, min(y0 + TFSF_YCH - 1, s.ny + 1));
+__global__ void __launch_bounds__(128) k_tfsf_table(SrcArgs s, int it0, const int* itp, int n, int ncol,
+                                                    TfsfVal<T>* __restrict__ out) {
+  const long j = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= (long)n * ncol) return;
+  if (itp) it0 += *itp;
+  out[j] = tfsf_entry<T>(s, it0 + (int)(j / ncol), (int)(j % ncol));
 }
 
+// One step's corrections, row: its table row.  One thread a cell of the
+// corrected planes (latency only: two reads and writes of a value each).
+template <typename T>
+__global__ void __launch_bounds__(256) k_tfsf(typename V2<T>::t* e, typename V2<T>::t* h, Geo g, SrcArgs s,
+                                              const TfsfVal<T>* __restrict__ row) {
+  const int ix = blockIdx.x * 64 + threadIdx.x, iy = blockIdx.y * 4 + threadIdx.y;
+  if (ix <= s.nx + 1 && iy <= s.ny + 1) tfsf_apply<T>(e, h, g, s, ix, iy, row[ix]);
+}
 
 template <typename T>
 __global__ void __launch_bounds__(256) k_dft_gather(const typename V2<T>::t* __restrict__ e,
@@ -1238,11 +1246,8 @@ FluxTiles flux_tiles(const FluxFace* f6) {
 //     any split gives the split passes' values; FP32 arithmetic may be
 //     contracted to FMAs differently in a different instantiation, so FP32
 //     keeps the split passes' own per-cell function, one item per cell;
-//   * the TF/SF corrections' incident field (exp, sincos and divisions in
-//     FP64, a dependent chain of a few hundred FP64 instructions) is
-//     evaluated for every step of the span up front by k_tfsf_table, in
-//     parallel; the TF/SF phase only adds the tabulated values, one thread
-//     per corrected row;
+//   * the TF/SF phase only adds the values that k_tfsf_table evaluates for
+//     every step of the span up front, one thread per corrected row;
 //   * the DFT sample reads a flat table of its points' field and storage
 //     index (one dependent load, not a walk over the run list), and shares
 //     the TF/SF phase (one barrier less a step) when no sample point lies on
@@ -1296,7 +1301,7 @@ __device__ __forceinline__ bool grid_barrier(GridBar* b, unsigned& target, unsig
 template <typename T> struct TinyArgs {
   FieldArgs<T> a;
   SrcArgs s;
-  const TfsfVal* tfv;    // TF/SF corrections per [step of the span][ix in 0..nx+1]
+  const TfsfVal<T>* tfv; // TF/SF corrections per [step of the span][ix in 0..nx+1]
   int merged;            // the DFT sample runs in the TF/SF phase
   const long* sidx;      // per sample point: storage index * 8 + field (0..5)
   const Seg* segs;
@@ -1323,16 +1328,6 @@ __global__ void k_barrier_check(GridBar* bar, int* err, int shift) {
   unsigned target = 0;
   if (blockIdx.x != 0) return;
   grid_barrier(bar, target, 2, err, STREAM_WAIT_CYCLES >> shift);
-}
-
-// The TF/SF corrections of steps it0 .. it0+n-1 for every column ix in
-// [0, nx+1] (tfsf_values, the split passes' function).
-__global__ void k_tfsf_table(SrcArgs s, int it0, int n, int ncol, TfsfVal* __restrict__ out) {
-  const long j = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= (long)n * ncol) return;
-  cx<double> vE, vH;
-  tfsf_values(s, it0 + (int)(j / ncol), (int)(j % ncol), vE, vH);
-  out[j] = TfsfVal{vE.re, vE.im, vH.re, vH.im};
 }
 
 // FP64 work items of k_tiny: component k of a cell, UPML cells with the slab
@@ -1435,8 +1430,7 @@ template <typename T, bool CEPS> __global__ void __launch_bounds__(TINY_MAX_THRE
     for (long w = gt; w < (one ? n_tf + n_s : n_tf); w += gs) {
       if (w < n_tf) {
         const int ix = (int)(w % (g.nx + 2)), iy = (int)(w / (g.nx + 2));
-        const TfsfVal v = A.tfv[(long)i * (g.nx + 2) + ix];
-        tfsf_apply<T>(A.a.e, A.a.h, g, A.s, ix, iy, iy, cx<double>{v.er, v.ei}, cx<double>{v.hr, v.hi});
+        tfsf_apply<T>(A.a.e, A.a.h, g, A.s, ix, iy, A.tfv[(long)i * (g.nx + 2) + ix]);
       } else {
         const long q = w - n_tf, code = A.sidx[q];
         const int f = (int)(code & 7);
@@ -1885,11 +1879,31 @@ template <typename T> void launch_h(iris_engine* E) {
   }
   k_update_h<T><<<E->grd, E->blk, 0, E->st>>>(field_args<T>(E));
 }
-template <typename T> void launch_tfsf(iris_engine* E, int it, const int* itp = nullptr) {
+// The TF/SF table of steps it .. it+n-1 (at most tfv_cap), from *itp on when
+// itp is given.
+template <typename T> void tfsf_table(iris_engine* E, int it, int n, const int* itp = nullptr) {
+  const int ncol = E->p.nx + 2;
+  k_tfsf_table<T><<<(unsigned)(((long)n * ncol + 127) / 128), 128, 0, E->st>>>(E->src, it, itp, n, ncol,
+                                                                              (TfsfVal<T>*)E->d_tfv);
+}
+
+// Step it's corrections; left: the steps the caller goes on to take, it
+// included.  The table is evaluated for as many of them as it holds whenever
+// the step lies outside the steps it covers (tf_at .. tf_end, reset by every
+// call that steps).
+template <typename T> void launch_tfsf(iris_engine* E, int it, int left, const int* itp = nullptr) {
   if (E->src.variant == 0) return;
   KTimer tm(E, IRIS_KC_TFSF);
   using V = typename V2<T>::t;
-  k_tfsf<T><<<E->tf_grd, E->tf_blk, 0, E->st>>>((V*)E->e, (V*)E->h, E->g, E->src, it, itp);
+  if (it < E->tf_at || it >= E->tf_end) {
+    const int n = std::max(1, std::min(left, E->tfv_cap));
+    tfsf_table<T>(E, it, n, itp);
+    E->tf_at = it;
+    E->tf_end = it + n;
+  }
+  const dim3 grd((unsigned)((E->p.nx + 2 + 63) / 64), (unsigned)((E->p.ny + 2 + 3) / 4));
+  k_tfsf<T><<<grd, dim3(64, 4), 0, E->st>>>((V*)E->e, (V*)E->h, E->g, E->src,
+                                            (const TfsfVal<T>*)E->d_tfv + (long)(it - E->tf_at) * (E->p.nx + 2));
 }
 
 template <typename T> void dft_sample(iris_engine* E, int t, const int* tp = nullptr) {
@@ -1943,8 +1957,8 @@ void fused_chunks(std::vector<int>& r, int za, int zb, long tiles) {
 
 // One fused step into the second buffers, swap, then TF/SF and the DFT
 // sample on the new state, in the operator order of the split passes; step
-// it, or *itp + it when itp is given.
-void fused_one(iris_engine* E, int it, const int* itp, bool sampled) {
+// it (left: the steps to take, it included), or *itp + it when itp is given.
+void fused_one(iris_engine* E, int it, int left, const int* itp, bool sampled) {
   {
     // the planes outside the UPML slabs with a kernel without slab code and,
     // concurrently on the second stream, the slabs: the two launches write
@@ -1989,7 +2003,7 @@ void fused_one(iris_engine* E, int it, const int* itp, bool sampled) {
   std::swap(E->e, E->e2);
   std::swap(E->h, E->h2);
   for (int s = 0; s < 2; ++s) std::swap(E->pml_d[s], E->pml_d2[s]);
-  launch_tfsf<float>(E, it, itp);
+  launch_tfsf<float>(E, it, left, itp);
   if (sampled) dft_sample<float>(E, it + 1 - E->p.to_fourier, itp);
 }
 
@@ -1999,13 +2013,15 @@ int step_fused(iris_engine* E, int it0, int n) {
   while (it < it0 + n) {
     if (graph_ready(E, it, it0 + n - it)) {
       int rc = graph_block(E, it, [&] {
-        for (int j = 0; j < E->K; ++j) fused_one(E, j, E->d_it, true);
+        E->tf_end = 0;
+        for (int j = 0; j < E->K; ++j) fused_one(E, j, E->K - j, E->d_it, true);
       });
+      E->tf_end = 0;
       if (rc) return rc;
       it += E->K;
       continue;
     }
-    fused_one(E, it, nullptr, it >= p.to_fourier && it % p.sample_fourier == 0);
+    fused_one(E, it, it0 + n - it, nullptr, it >= p.to_fourier && it % p.sample_fourier == 0);
     ++it;
   }
   CK(cudaGetLastError());
@@ -2018,20 +2034,22 @@ template <typename T> int step_t(iris_engine* E, int it0, int n) {
   while (it < it0 + n) {
     if (graph_ready(E, it, it0 + n - it)) {
       int rc = graph_block(E, it, [&] {
+        E->tf_end = 0;
         for (int j = 0; j < E->K; ++j) {
           launch_e<T>(E);
           launch_h<T>(E);
-          launch_tfsf<T>(E, j, E->d_it);
+          launch_tfsf<T>(E, j, E->K - j, E->d_it);
           dft_sample<T>(E, j + 1 - p.to_fourier, E->d_it);
         }
       });
+      E->tf_end = 0;
       if (rc) return rc;
       it += E->K;
       continue;
     }
     launch_e<T>(E);
     launch_h<T>(E);
-    launch_tfsf<T>(E, it);
+    launch_tfsf<T>(E, it, it0 + n - it);
     if (it >= p.to_fourier && it % p.sample_fourier == 0) dft_sample<T>(E, it + 1 - p.to_fourier);
     ++it;
   }
@@ -2060,6 +2078,187 @@ static bool tiny_sample_merges(const iris_engine* E) {
   return true;
 }
 
+// The kernel of a resident engine.
+template <typename T> const void* res_kernel(const iris_engine* E, bool cplx) {
+  if (E->res_nc == 6) return cplx ? (const void*)k_res<T, true, 6> : (const void*)k_res<T, false, 6>;
+  return cplx ? (const void*)k_res<T, true, 5> : (const void*)k_res<T, false, 5>;
+}
+
+// Row ranges of the resident kernel's CTAs: R rows over G CTAs, a UPML row
+// weighing w interior rows; the widest range in rows.
+int res_partition(const iris_params& p, int G, double w, std::vector<ResCta>& out) {
+  const long R = (long)p.ny * p.nz;
+  auto weight = [&](long r) {
+    const long z = r / p.ny + 1;
+    return z <= p.pmlzi || z >= p.pmlzf ? w : 1.0;
+  };
+  double tot = 0.0;
+  for (long r = 0; r < R; ++r) tot += weight(r);
+  out.assign(G, ResCta{});
+  long r = 0;
+  double cum = 0.0;
+  int widest = 0;
+  for (int c = 0; c < G; ++c) {
+    out[c].r0 = (int)r;
+    const double end = tot * (c + 1) / G;
+    // at least one row each, and one left for every CTA after this one
+    while (r < R - (G - 1 - c) && (r == out[c].r0 || c == G - 1 || cum + 0.5 * weight(r) <= end)) cum += weight(r++);
+    out[c].r1 = (int)r;
+    widest = std::max(widest, out[c].r1 - out[c].r0);
+  }
+  // neighbours: the owners of the ny rows before and after, cyclically
+  std::vector<int> owner(R);
+  for (int c = 0; c < G; ++c)
+    for (int q = out[c].r0; q < out[c].r1; ++q) owner[q] = c;
+  for (int c = 0; c < G; ++c) {
+    int before = 0, after = 0;
+    for (long d = 1; d <= p.ny; ++d) {
+      const int lo = owner[((out[c].r0 - d) % R + R) % R], hi = owner[(out[c].r1 - 1 + d) % R];
+      before = std::max(before, ((c - lo) % G + G) % G);
+      after = std::max(after, ((hi - c) % G + G) % G);
+    }
+    const int n = std::min(G - 1, before + after);
+    out[c].nb0 = n == G - 1 ? (c + 1) % G : ((c - before) % G + G) % G;
+    out[c].nbn = n == G - 1 ? n : n + 1;  // the CTA itself lies between and has always arrived
+  }
+  return widest;
+}
+
+// Whether a persistent engine's state fits in shared memory and its TF/SF
+// corrections have the form k_res applies; sets its launch up.
+int res_setup(iris_engine* E) {
+  const iris_params& p = E->p;
+  const SrcArgs& s = E->src;
+  if (p.nx >= 65536 - 64 || p.ny >= 65536 || p.nz >= 32768) return IRIS_OK;
+  ResSrc q{};
+  const bool one_y = E->ph[1][0] == 1.0 && E->ph[1][1] == 0.0 && E->ph[4][0] == 1.0 && E->ph[4][1] == 0.0;
+  if (s.variant != 0) {
+    q.on = 1;
+    const bool pol2 = s.variant == 2 || s.i_pol == 2;
+    q.cE = pol2 ? 0 : 1;
+    q.cH = pol2 ? 1 : 0;
+    q.zE = s.iz_min;
+    q.zH = s.variant == 1 ? s.iz_min - 1 : s.iz_min;
+    q.sgn = pol2 ? 1 : -1;
+    q.gx = s.variant == 2 || !pol2;
+    q.gy = s.variant == 2 || pol2;
+    // images across z would carry a correction, and with an H_x correction
+    // so would the y images (exact only where the phase is 1)
+    if (q.zH < 1 || q.zE < 2 || q.zE > p.nz - 1 || (q.cH == 0 && !one_y)) return IRIS_OK;
+  }
+  int nsm = 0, optin = 0;
+  CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, E->device));
+  CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, E->device));
+  const long R = (long)p.ny * p.nz;
+  const int G = (int)std::min<long>(nsm, R);
+  // the fewest rows any partition has must fit before the partitions are tried
+  const size_t row5 = 5 * (size_t)(p.nx + 2) * E->esz;
+  if ((size_t)((R + G - 1) / G) * row5 > (size_t)optin) return IRIS_OK;
+  // Ranges weighted by time, a UPML row costing about 2.5 others in FP64 (its
+  // arithmetic) and 2 in FP32; by memory (twice the components) when those do
+  // not fit; D and B left in their global arrays when neither does.
+  const double w = E->prec == IRIS_FP64 ? 2.5 : 2.0;
+  const size_t rsz = E->esz / 2;
+  // warps take 32-cell runs of rows where at most a third of the lanes idle
+  E->res_runs = E->prec == IRIS_FP32 && 3 * p.nx >= 2 * ((p.nx + 31) / 32 * 32);
+  bool fits = false;
+  for (int t = 0; t < 6 && !fits; ++t) {
+    const int nc = t < 2 || t == 4 ? 6 : 5, db = t < 4;
+    const double wt = !db ? 1.0 : t % 2 == 0 ? w : (nc + 6.0) / nc;
+    const int rows = res_partition(p, G, wt, E->res_cta);
+    const int nruns = E->res_runs ? rows * ((p.nx + 31) / 32) : 0;
+    // (the fields behind the tables are 16-byte aligned)
+    const size_t head = ((2 * sizeof(ResRow) + sizeof(uint2)) * rows + 2 * sizeof(unsigned) * nruns + 15) / 16 * 16;
+    size_t most = 0, items = 0;
+    for (const ResCta& c : E->res_cta) {
+      size_t nu = 0;
+      for (long r = c.r0; r < c.r1; ++r) nu += r / p.ny < p.pmlzi || r / p.ny + 1 >= p.pmlzf;
+      const size_t n = c.r1 - c.r0;
+      most = std::max(most, n * (p.nx + 2) * nc * E->esz + (db ? nu * (6 * p.nx * E->esz + NCOEF * rsz) : 0));
+      items = std::max(items, n * p.nx * (E->prec == IRIS_FP64 ? 6 : 1));
+    }
+    if (head + most + 512 > (size_t)optin) continue;  // 512: the kernel's static shared memory, rounded up
+    E->res_nc = nc;
+    E->res_db = db;
+    E->res_rows = rows;
+    E->res_nruns = nruns;
+    E->res_head = (int)head;
+    E->res_smem = head + most;
+    E->res_threads = (int)std::min<size_t>(RES_THREADS, std::max<size_t>(64, (items + 31) / 32 * 32));
+    fits = true;
+  }
+  if (!fits) return IRIS_OK;
+  E->res_blocks = G;
+  E->res_src = q;
+  for (int cplx = 0; cplx < 2; ++cplx) {
+    const void* k = E->prec == IRIS_FP64 ? res_kernel<double>(E, cplx) : res_kernel<float>(E, cplx);
+    int occ = 0;
+    CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - 512));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, E->res_threads, E->res_smem));
+    if (occ < 1) return IRIS_OK;
+  }
+  CK(cudaMalloc(&E->d_rcta, sizeof(ResCta) * G));
+  CK(cudaMalloc(&E->d_rflag, sizeof(unsigned) * RES_FLAG_STRIDE * G));
+  E->res = true;
+  return IRIS_OK;
+}
+
+// The sample points of every CTA, E then H, each in ring order: shared-memory
+// offset (E_x outside it: storage index) with its flags, and ring position.
+int res_samples(iris_engine* E) {
+  const Geo& g = E->g;
+  const int W = g.nx + 2, G = E->res_blocks;
+  std::vector<int> owner((size_t)g.ny * g.nz);
+  for (int c = 0; c < G; ++c)
+    for (int q = E->res_cta[c].r0; q < E->res_cta[c].r1; ++q) owner[q] = c;
+  // points of one face run advance by one cell in x (su = 1) or one row
+  // (su = pitch); its v axis by one row or one plane of rows
+  std::vector<unsigned> at(2 * (size_t)G + 1, 0);
+  auto start = [&](const Seg& sg, int& x, int& row) {
+    const int z = (int)(sg.src / g.plane), in = (int)(sg.src - (long)z * g.plane), y = in / (int)g.pitch;
+    x = in - y * (int)g.pitch - g.xo;
+    row = (z - 1) * g.ny + y - 1;
+  };
+  for (const Seg& sg : E->segs) {
+    const int h = sg.field >= 3, dv = sg.sv == g.plane ? g.ny : 1;
+    int x, row;
+    start(sg, x, row);
+    for (int v = 0; v < sg.nv; ++v, row += dv) {
+      if (sg.su == 1) at[2 * owner[row] + h + 1] += sg.nu;
+      else
+        for (int u = 0; u < sg.nu; ++u) ++at[2 * owner[row + u] + h + 1];
+    }
+  }
+  for (size_t i = 1; i < at.size(); ++i) at[i] += at[i - 1];
+  for (int c = 0; c < G; ++c) {
+    E->res_cta[c].s0 = at[2 * c];
+    E->res_cta[c].sh = at[2 * c + 1];
+    E->res_cta[c].s1 = at[2 * c + 2];
+  }
+  std::vector<uint2> tab((size_t)std::max(1L, E->P));
+  for (const Seg& sg : E->segs) {
+    const int h = sg.field >= 3, dv = sg.sv == g.plane ? g.ny : 1;
+    const bool global = E->res_nc == 5 && sg.field == 0;
+    const bool corr = !h && E->res_src.on && sg.field == E->res_src.cE;
+    int x, row;
+    start(sg, x, row);
+    unsigned pos = (unsigned)sg.p0;
+    for (int v = 0; v < sg.nv; ++v, row += dv)
+      for (int u = 0; u < sg.nu; ++u, ++pos) {
+        const int r = sg.su == 1 ? row : row + u, xx = sg.su == 1 ? x + u : x;
+        const ResCta& c = E->res_cta[owner[r]];
+        unsigned off = global ? (unsigned)(sg.src + u * sg.su + v * sg.sv) | RES_GLOBAL
+                              : (unsigned)(((sg.field - (6 - E->res_nc)) * (c.r1 - c.r0) + r - c.r0) * W + xx);
+        if (corr && r / g.ny + 1 == E->res_src.zE) off |= RES_CORR;
+        tab[at[2 * owner[r] + h]++] = make_uint2(off, pos);
+      }
+  }
+  CK(cudaMalloc(&E->d_rsamp, sizeof(uint2) * tab.size()));
+  CK(cudaMemcpy(E->d_rsamp, tab.data(), sizeof(uint2) * tab.size(), cudaMemcpyHostToDevice));
+  CK(cudaMemcpy(E->d_rcta, E->res_cta.data(), sizeof(ResCta) * G, cudaMemcpyHostToDevice));
+  return IRIS_OK;
+}
+
 // Steps it0 .. it0+n-1 with the persistent kernel: spans that end where the
 // DFT ring fills (its commit runs between launches), after 1024 steps or at
 // the TF/SF table's capacity; before each span k_tfsf_table evaluates its
@@ -2067,8 +2266,10 @@ static bool tiny_sample_merges(const iris_engine* E) {
 template <typename T> int step_persist(iris_engine* E, int it0, int n) {
   const iris_params& p = E->p;
   const int cap = E->src.variant != 0 ? E->tfv_cap : 1024;
-  const bool merged = tiny_sample_merges(E);
-  if (E->P > 0 && !E->d_sidx) {
+  const bool merged = !E->res && tiny_sample_merges(E);
+  if (E->res && !E->d_rsamp)
+    if (int rc = res_samples(E)) return rc;
+  if (!E->res && E->P > 0 && !E->d_sidx) {
     // flat table of the sample points: storage index * 8 + field
     std::vector<long> code((size_t)E->P);
     for (const Seg& sg : E->segs)
@@ -2090,7 +2291,7 @@ template <typename T> int step_persist(iris_engine* E, int it0, int n) {
     TinyArgs<T> A{};
     A.a = field_args<T>(E);
     A.s = E->src;
-    A.tfv = E->d_tfv;
+    A.tfv = (const TfsfVal<T>*)E->d_tfv;
     A.merged = merged ? 1 : 0;
     A.sidx = E->d_sidx;
     A.segs = E->d_segs;
@@ -2109,13 +2310,42 @@ template <typename T> int step_persist(iris_engine* E, int it0, int n) {
     void* args[] = {&A};
     {
       KTimer tm(E, IRIS_KC_PERSIST);
-      if (E->src.variant != 0) {
-        const long nt = (long)span * (p.nx + 2);
-        k_tfsf_table<<<(unsigned)((nt + 127) / 128), 128, 0, E->st>>>(E->src, it, span, p.nx + 2, E->d_tfv);
+      if (E->src.variant != 0) tfsf_table<T>(E, it, span);
+      if (E->res) {
+        ResArgs<T> B{};
+        B.a = A.a;
+        B.s = E->res_src;
+        B.tfv = A.tfv;
+        B.cta = E->d_rcta;
+        B.samp = E->d_rsamp;
+        B.S = A.S;
+        B.P = E->P;
+        B.tk = E->d_tk;
+        B.slot0 = E->nslot;
+        B.it0 = it;
+        B.n = span;
+        B.to_fourier = p.to_fourier;
+        B.sample_fourier = p.sample_fourier;
+        B.dft = A.dft;
+        B.db = E->res_db;
+        B.rows = E->res_rows;
+        B.head = E->res_head;
+        B.runs = E->res_runs;
+        B.nruns = E->res_nruns;
+        for (int k = 0; k < 3; ++k)
+          B.one[k] = E->ph[k][0] == 1.0 && E->ph[k][1] == 0.0 && E->ph[3 + k][0] == 1.0 && E->ph[3 + k][1] == 0.0;
+        B.flag = E->d_rflag;
+        B.err = E->d_err;
+        long long limit = STREAM_WAIT_CYCLES;
+        void* rargs[] = {&B, &limit};
+        CK(cudaMemsetAsync(E->d_rflag, 0, sizeof(unsigned) * RES_FLAG_STRIDE * E->res_blocks, E->st));
+        CK(cudaLaunchCooperativeKernel(res_kernel<T>(E, E->eps_complex), dim3(E->res_blocks), dim3(E->res_threads),
+                                       rargs, E->res_smem, E->st));
+      } else {
+        CK(cudaMemsetAsync(E->d_bar, 0, sizeof(GridBar), E->st));
+        const void* k = E->eps_complex ? (const void*)k_tiny<T, true> : (const void*)k_tiny<T, false>;
+        CK(cudaLaunchCooperativeKernel(k, dim3(E->persist_blocks), dim3(E->persist_threads), args, 0, E->st));
       }
-      CK(cudaMemsetAsync(E->d_bar, 0, sizeof(GridBar), E->st));
-      const void* k = E->eps_complex ? (const void*)k_tiny<T, true> : (const void*)k_tiny<T, false>;
-      CK(cudaLaunchCooperativeKernel(k, dim3(E->persist_blocks), dim3(E->persist_threads), args, 0, E->st));
     }
     E->nslot += samples;
     if (E->nslot == E->K) dft_flush(E);
@@ -2508,7 +2738,7 @@ void free_engine(iris_engine* E) {
   void* ptrs[] = {E->e, E->h, E->pml_d[0], E->pml_d[1], E->pml_b[0], E->pml_b[1], E->coef, E->eps, E->d_segs,
                   E->S, E->d_tk, E->d_fw, E->fd, E->d_wt, E->d_faces, E->d_J, E->e2, E->h2, E->pml_d2[0],
                   E->pml_d2[1], E->d_err, E->d_it, E->d_wtc, E->d_wt64, E->d_part, E->d_bar, E->d_stage,
-                  E->d_tfv, E->d_sidx};
+                  E->d_tfv, E->d_sidx, E->d_rcta, E->d_rsamp, E->d_rflag};
   for (void* q : ptrs)
     if (q) cudaFree(q);
   if (E->h_J) cudaFreeHost(E->h_J);
@@ -2527,20 +2757,20 @@ void free_engine(iris_engine* E) {
 }
 
 
-void one_step(iris_engine* E, int it, bool dft) {
+void one_step(iris_engine* E, int it, int left, bool dft) {
   const iris_params& p = E->p;
   const bool sampled = dft && it >= p.to_fourier && it % p.sample_fourier == 0;
   if (E->fused) {
-    fused_one(E, it, nullptr, sampled);
+    fused_one(E, it, left, nullptr, sampled);
   } else if (E->prec == IRIS_FP64) {
     launch_e<double>(E);
     launch_h<double>(E);
-    launch_tfsf<double>(E, it);
+    launch_tfsf<double>(E, it, left);
     if (sampled) dft_sample<double>(E, it + 1 - p.to_fourier);
   } else {
     launch_e<float>(E);
     launch_h<float>(E);
-    launch_tfsf<float>(E, it);
+    launch_tfsf<float>(E, it, left);
     if (sampled) dft_sample<float>(E, it + 1 - p.to_fourier);
   }
 }
@@ -2629,8 +2859,6 @@ int create_engine(const iris_params* pin, const double* fw, bool member, bool z_
   E->blk = dim3(bx, by, bz);
   E->grd = dim3((p.nx + bx - 1) / bx, (p.ny + by - 1) / by, (p.nz + bz - 1) / bz);
   E->src = make_src(p);
-  E->tf_blk = dim3(64);
-  E->tf_grd = dim3((p.nx + 2 + 63) / 64, (p.ny + 2 + TFSF_YCH - 1) / TFSF_YCH);
   // Small grids step with the persistent kernel (asked for, or by default
   // when the device runs cooperative launches: FP64 grids of at most
   // IRIS_PERSISTENT_MAX_CELLS cells, FP32 grids of at most
@@ -2671,12 +2899,16 @@ int create_engine(const iris_params* pin, const double* fw, bool member, bool z_
                                     "fewer than 2^31 / 3 cells"));
     if (E->persist && cudaMalloc(&E->d_bar, 64) != cudaSuccess)
       return bail(fail(IRIS_ENOMEM, "barrier allocation failed"));
-    if (E->persist && E->src.variant != 0) {
+    if (!member && E->src.variant != 0) {
       // TF/SF table of a span: at most 1024 steps and 8 MB
       E->tfv_cap = (int)std::max(1L, std::min(1024L, (8L << 20) / (32L * (p.nx + 2))));
-      if (cudaMalloc(&E->d_tfv, sizeof(TfsfVal) * (size_t)E->tfv_cap * (p.nx + 2)) != cudaSuccess)
+      if (cudaMalloc(&E->d_tfv, sizeof(TfsfVal<double>) * (size_t)E->tfv_cap * (p.nx + 2)) != cudaSuccess)
         return bail(fail(IRIS_ENOMEM, "TF/SF table allocation failed"));
     }
+  }
+  if (E->persist) {
+    rc = res_setup(E);
+    if (rc) return bail(rc);
   }
   E->fused = !E->persist && E->prec == IRIS_FP32 &&
              (p.stencil == IRIS_STENCIL_FUSED || (p.stencil == IRIS_STENCIL_DEFAULT && fused_fill(p.nx, p.ny) >= 0.5));
@@ -2922,6 +3154,7 @@ int iris_step(iris_engine* E, int it0, int nsteps) {
   clear_error();
   if (!E || nsteps < 0) return fail(IRIS_EINVAL, "bad argument");
   CK(cudaSetDevice(E->device));
+  E->tf_end = 0;
   if (E->persist)
     return E->prec == IRIS_FP64 ? step_persist<double>(E, it0, nsteps) : step_persist<float>(E, it0, nsteps);
   if (E->fused) return step_fused(E, it0, nsteps);
@@ -3278,7 +3511,10 @@ int iris_apply(iris_engine* E, int op, int arg) {
   switch (op) {
     case IRIS_OP_E: d ? launch_e<double>(E) : launch_e<float>(E); break;
     case IRIS_OP_H: d ? launch_h<double>(E) : launch_h<float>(E); break;
-    case IRIS_OP_TFSF: d ? launch_tfsf<double>(E, arg) : launch_tfsf<float>(E, arg); break;
+    case IRIS_OP_TFSF:
+      E->tf_end = 0;
+      d ? launch_tfsf<double>(E, arg, 1) : launch_tfsf<float>(E, arg, 1);
+      break;
     case IRIS_OP_DFT:
       dft_flush(E);
       d ? dft_sample<double>(E, arg) : dft_sample<float>(E, arg);

@@ -14,6 +14,7 @@
 
 #include "iris_device.cuh"
 #include "iris_internal.h"
+#include "iris_resident.cuh"
 
 // Return IRIS_ECUDA (IRIS_ENOMEM for an allocation) with the failing call's
 // text when a CUDA runtime call fails.
@@ -57,7 +58,6 @@ struct iris_engine {
   bool eps_complex = false;
   double ph[6][2] = {};  // exp(+i akx), exp(+i aky), exp(+i akz), exp(-i akx), ...
   iris::SrcArgs src{};
-  dim3 tf_blk, tf_grd;
   // DFT
   int nboxes = 1;
   iris::FaceMap fm[2][3];
@@ -118,10 +118,21 @@ struct iris_engine {
   bool persist = false;
   int persist_blocks = 0, persist_threads = 0;
   void* d_bar = nullptr;
-  // its TF/SF corrections (vE, vH) per [step of a span][ix], up to tfv_cap steps
-  iris::TfsfVal* d_tfv = nullptr;
-  int tfv_cap = 0;
+  // TF/SF corrections (iris::TfsfVal) per [step][ix], up to tfv_cap steps; outside
+  // the persistent kernels: the steps tf_at .. tf_end - 1 it holds within a call
+  void* d_tfv = nullptr;
+  int tfv_cap = 0, tf_at = 0, tf_end = 0;
   long* d_sidx = nullptr;  // its DFT sample points: storage index * 8 + field
+  // the resident form of it (k_res): grids whose E and H fit in shared memory
+  bool res = false;
+  bool res_runs = false;
+  int res_nc = 6, res_db = 1, res_rows = 0, res_nruns = 0, res_head = 0, res_blocks = 0, res_threads = 0;
+  size_t res_smem = 0;
+  iris::ResSrc res_src{};
+  std::vector<iris::ResCta> res_cta;  // row ranges and neighbours per CTA
+  iris::ResCta* d_rcta = nullptr;
+  uint2* d_rsamp = nullptr;
+  unsigned* d_rflag = nullptr;
   // staging buffer of the complex(8) field transfers (allocated on first use)
   void* d_stage = nullptr;
   size_t stage_bytes = 0;
@@ -218,8 +229,9 @@ int fd_materialise(iris_engine* E);
 int read_flux(iris_engine* E, int set, double* J);
 // One step (the fused pass or the split E and H passes, as the engine
 // steps, then TF/SF), with the DFT sample of step it when dft is set and the
-// step is sampled.
-void one_step(iris_engine* E, int it, bool dft);
+// step is sampled; left: the steps the caller goes on to take, it included
+// (the caller resets tf_end before the first).
+void one_step(iris_engine* E, int it, int left, bool dft);
 
 // Bounds-check records of the batch and adjoint modules (read and cleared;
 // 0 in the ordinary build).
