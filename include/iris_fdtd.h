@@ -40,7 +40,9 @@ extern "C" {
 #define IRIS_ENODEV (-8)   /* no CUDA device                                 */
 
 /* ---- precision modes ------------------------------------------------ */
-/* FP64 fields and DFT, operations in the reference's order (parity mode). */
+/* FP64 fields, operations in the reference's order (parity mode); FP64 DFT,
+ * a block's partial sums formed to 2^-56 of the point's largest sample and
+ * added to fdata with one rounding.                                        */
 #define IRIS_FP64 0
 /* FP32 fields; TF/SF incident field in FP64; DFT partial sums over a block
  * of K samples in FP32 with FP64-exact twiddles, accumulated in FP64.     */
@@ -264,8 +266,8 @@ int iris_sync(iris_engine* eng);
  * major: the Jabs array of scattering_fourier_out
  * (code/dataprocess.f90:243-277), eps0*Q/(2 dt) included.  Returns
  * IRIS_ENAN if any value is not finite.  Every sample taken so far counts;
- * in IRIS_FP32 mode (tensor-core DFT) the samples still buffered are added
- * on the fly and stay buffered, so a flux read changes no state.
+ * the samples still buffered are added on the fly and stay buffered (except
+ * with IRIS_DFT_KERNEL_CUDA), so a flux read changes no state.
  */
 int iris_flux(iris_engine* eng, int box, double* J);
 

@@ -22,6 +22,7 @@
 // iris_adjoint.cu; the per-cell operators they share are in iris_device.cuh,
 // the fused pass's tile column in iris_fused.cuh.
 
+#include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -420,56 +421,6 @@ __global__ void __launch_bounds__(256) k_dft_gather(const typename V2<T>::t* __r
   gather_run<T>(sg, src, slot, comp, np);
 }
 
-// FP64 mode: fdata(p, iw) += (dt*F_k(p))*exp(i*fw(iw)*t_k), k in the
-// reference's order (code/dataprocess.f90:143-147), each complex
-// multiply-add as four FP64 FMAs (GB300's FP64 rate makes the unfused eight
-// operations the cost of the FP64 mode; the difference is one rounding per
-// term).  The twiddles exp(i*fw*t_k) come from one table per block.
-constexpr int DFT64_WC = 8;
-__global__ void k_twiddle64(const int* __restrict__ tk, int nk, const double* __restrict__ fw, int nof,
-                            double2* __restrict__ W) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nk * nof) return;
-  const int k = t / nof, j = t % nof;
-  double sn, cs;
-  sincos(dm(fw[j], (double)tk[k]), &sn, &cs);
-  W[t] = make_double2(cs, sn);
-}
-
-__global__ void __launch_bounds__(128) k_dft_fp64(const double2* __restrict__ S, long P, int nk,
-                                                  const double2* __restrict__ W, int nof, int nwc, double dt,
-                                                  double2* __restrict__ fd) {
-  extern __shared__ double2 W64[];  // [nk][WC]
-  // 1-D grid, frequency chunks fastest: the chunks of one point block share its samples in L2
-  const int w0 = (blockIdx.x % nwc) * DFT64_WC;
-  const long pblk = blockIdx.x / nwc;
-  for (int t = threadIdx.x; t < nk * DFT64_WC; t += blockDim.x) {
-    const int k = t / DFT64_WC, j = t % DFT64_WC;
-    W64[t] = w0 + j < nof ? W[(long)k * nof + w0 + j] : make_double2(0.0, 0.0);
-  }
-  __syncthreads();
-  const long p = pblk * blockDim.x + threadIdx.x;
-  if (p >= P) return;
-  const int nw = min(DFT64_WC, nof - w0);
-  double2 acc[DFT64_WC];
-#pragma unroll
-  for (int j = 0; j < DFT64_WC; ++j)
-    if (j < nw) acc[j] = fd[(long)(w0 + j) * P + p];
-  for (int k = 0; k < nk; ++k) {
-    const double2 f = S[(long)k * P + p];
-    const double ar = dm(dt, f.x), ai = dm(dt, f.y);
-#pragma unroll
-    for (int j = 0; j < DFT64_WC; ++j) {
-      const double2 w = W64[k * DFT64_WC + j];
-      acc[j].x = fma(ar, w.x, fma(-ai, w.y, acc[j].x));
-      acc[j].y = fma(ar, w.y, fma(ai, w.x, acc[j].y));
-    }
-  }
-#pragma unroll
-  for (int j = 0; j < DFT64_WC; ++j)
-    if (j < nw) fd[(long)(w0 + j) * P + p] = acc[j];
-}
-
 // FP32 mode accumulators: each complex value of fdata is a compensated
 // (double-float) pair per part, float4 (re_hi, im_hi, re_lo, im_lo), 16 bytes
 // like a double2.  GB300 runs FP64 arithmetic at a small fraction of its FP32
@@ -837,7 +788,7 @@ template <bool FLUX> struct WsRow {
   int nl, tile;
 };
 
-template <bool FLUX> __device__ __forceinline__ WsRow<FLUX> ws_item(const WsArgs& A, long item, int& g) {
+template <bool FLUX, typename ARGS> __device__ __forceinline__ WsRow<FLUX> ws_item(const ARGS& A, long item, int& g) {
   WsRow<FLUX> r{};
   g = (int)(item % A.ngroups);
   const long t = item / A.ngroups;
@@ -1189,6 +1140,344 @@ template <bool FLUX> __device__ __forceinline__ void dft_ws(const WsArgs& A) {
 
 __global__ void __maxnreg__(80) k_dft_ws_commit(WsArgs A) { dft_ws<false>(A); }
 __global__ void __launch_bounds__(WsCfg<true>::THREADS, 1) k_dft_ws_flux(WsArgs A) { dft_ws<true>(A); }
+
+// ---------------------------------------------------------------------------
+// FP64 DFT block on the tensor cores (tcgen05.mma kind::f16, exact slices).
+//
+// fdata[iw][p] += sum_k F_k(p) dt exp(i fw(iw) t_k) in FP64 is 4 FP64 FMAs a
+// (point, frequency, sample), and GB300 runs two a cycle per SM: it took as
+// long as the FP64 stencil.  Here the products are integer ones that the bf16
+// tensor cores form exactly (the splitting of Ozaki et al., Numer. Algorithms
+// 59, 2012, with a common scale per row):
+//   * over a block of up to D64_S samples every point's values are written as
+//     X 2^(e-55), X an integer of at most 55 bits and 2^e the power of two
+//     above the row's largest magnitude, every twiddle likewise with one
+//     exponent for all; X is cut into D64_D = 7 balanced digits of 8 bits,
+//     which bf16 holds exactly;
+//   * the digit products of equal weight (digits s and t, s + t = o) are
+//     summed by the tensor cores in one FP32 accumulator per order o = 0..7:
+//     at most 7 pairs x 64 terms x 2^14 < 2^23, so every partial sum is an
+//     integer that FP32 holds exactly.  Orders above 7 lie below 2^-63 of the
+//     largest product and are left out;
+//   * the epilogue adds the eight integers with their weights in 64-bit
+//     integer arithmetic, rounds the sum to FP64 once and adds it to fdata
+//     with one FP64 add per number (two cycles a pair of lanes instead of 128).
+// A digit split is off by 2^-56 of the row's largest sample, a chain of FMAs
+// by 2^-53 of each partial sum.  A row with a value that is not finite gives
+// NaN.
+//
+// A work item is 128 points (the TMEM lanes) and a group of 32 frequencies (64
+// columns x 8 orders = all 512 TMEM columns); a CTA takes a run of items with
+// the groups of a tile next to each other, so a tile's digits are cut once.
+// Everything of an item is in shared memory (A 112 KB, B 56 KB): load,
+// MMAs and epilogue follow each other, B of the next item loading meanwhile.
+
+constexpr int D64_M = 128, D64_F = 32, D64_N = 2 * D64_F, D64_S = 32, D64_K = 2 * D64_S, D64_D = 7, D64_O = 8;
+constexpr int D64_A = D64_M * D64_K, D64_B = D64_N * D64_K;  // elements of one digit plane
+constexpr int D64_THREADS = 512;
+constexpr size_t D64_SMEM = 2 * (size_t)D64_D * (D64_A + D64_B);
+
+// Offset of element (row r, k) of a K-major, unswizzled bf16 operand of D64_K
+// columns: 8-row x 16-byte core matrices, the next 8 columns 128 bytes on.
+__host__ __device__ __forceinline__ int d64_off(int r, int k) {
+  return ((r >> 3) * (D64_K / 8) + (k >> 3)) * 64 + (r & 7) * 8 + (k & 7);
+}
+__device__ __forceinline__ uint64_t d64_desc(const void* smem) {
+  const uint64_t a = (smem_u32(smem) & 0x3FFFFu) >> 4;
+  const uint64_t lbo = 128u >> 4, sbo = (uint64_t)(D64_K / 8 * 128) >> 4;
+  return a | (lbo << 16) | (sbo << 32) | (1ull << 46);
+}
+__device__ __forceinline__ void d64_mma(uint32_t d_tmem, uint64_t a, uint64_t b, int acc) {
+  // D = F32, A = B = BF16, both K-major, M = 128, N = D64_N
+  constexpr uint32_t idesc =
+      (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(D64_N >> 3) << 17) | ((uint32_t)(D64_M >> 4) << 24);
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem),
+      "l"(a), "l"(b), "r"(idesc), "r"(acc)
+      : "memory");
+}
+
+// x as the integer X of x = X 2^(emax - 1022 - 55), emax the row's largest
+// biased exponent; rounded to nearest.
+__device__ __forceinline__ long long d64_int(double x, int emax) {
+  const unsigned long long u = (unsigned long long)__double_as_longlong(x);
+  int e = (int)(u >> 52) & 0x7ff;
+  unsigned long long m = u & 0xfffffffffffffull;
+  if (e) m |= 1ull << 52;
+  else e = 1;
+  const int r = emax - e - 2;
+  if (r <= 0) m <<= -r;
+  else m = r > 54 ? 0ull : (m + (1ull << (r - 1))) >> r;
+  return (u >> 63) ? -(long long)m : (long long)m;
+}
+// The D64_D digits of X, most significant first, as bf16 bits in the low half
+// of d[s].
+__device__ __forceinline__ void d64_digits(long long X, unsigned d[D64_D]) {
+#pragma unroll
+  for (int s = D64_D - 1; s >= 0; --s) {
+    const int v = s ? (int)(signed char)(X & 0xff) : (int)X;
+    // |v| <= 128: the float 1.5 2^23 + v holds v in its low bits
+    d[s] = __float_as_uint(__fsub_rn(__uint_as_float(0x4B400000u + (unsigned)v), 12582912.0f)) >> 16;
+    X = (X - v) >> 8;
+  }
+}
+
+// Twiddles dt exp(i fw t_k) of nk samples as B operands: sub-block, group g,
+// digit s, row n = 2 j + d (frequency 32 g + j), column 2 k + c, the real 2 x 2 form of
+// the complex product.  eb: biased exponent of their common scale (dt's).
+__global__ void __launch_bounds__(256) k_twiddle_d64(const int* __restrict__ tk, int nk, const double* __restrict__ fw,
+                                                     int nof, double dt, int ngroups, __nv_bfloat16_raw* __restrict__ Bt) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;  // (sub-block, group, frequency, sample)
+  const int kk = t % D64_S, j = (t / D64_S) % D64_F, sg = t / (D64_S * D64_F), g = sg % ngroups, iw = g * D64_F + j;
+  const int k = sg / ngroups * D64_S + kk;
+  if (k - kk >= nk) return;
+  double wr = 0.0, wi = 0.0;
+  if (iw < nof && k < nk) {
+    double sn, cs;
+    sincos(dm(fw[iw], (double)tk[k]), &sn, &cs);
+    wr = dm(dt, cs);
+    wi = dm(dt, sn);
+  }
+  const int eb = (int)((unsigned long long)__double_as_longlong(dt) >> 52) & 0x7ff;
+  unsigned dr[D64_D], di[D64_D], dn[D64_D];
+  const long long xi = d64_int(wi, eb);
+  d64_digits(d64_int(wr, eb), dr);
+  d64_digits(xi, di);
+  d64_digits(-xi, dn);
+#pragma unroll
+  for (int s = 0; s < D64_D; ++s) {
+    unsigned* b = (unsigned*)(Bt + ((long)sg * D64_D + s) * D64_B);
+    b[d64_off(2 * j, 2 * kk) / 2] = dr[s] | (dn[s] << 16);      // Re: wr, -wi
+    b[d64_off(2 * j + 1, 2 * kk) / 2] = di[s] | (dr[s] << 16);  // Im: wi, wr
+  }
+}
+
+struct D64Args {
+  const double2* S;  // the samples [nk][P]
+  long P;
+  int nk, nsb;       // samples, sub-blocks of D64_S of them
+  const __nv_bfloat16_raw* Bt;  // [sub-block][group][digit][D64_B]
+  double2* fd;       // [nof][P]
+  int fd_zero;       // fd holds no sum yet: written without being read
+  int nof, ngroups, eb;
+  long nitems;
+  // flux mode
+  const FluxFace* faces;
+  FluxTiles ft;
+  double* part;
+  int* err;
+};
+
+// The double nearest V 2^e (round half away from zero; 0 below the normal
+// range), formed with integer operations.
+__device__ __forceinline__ double d64_value(long long V, int e) {
+  if (V == 0) return 0.0;
+  unsigned long long m = V < 0 ? 0ull - (unsigned long long)V : (unsigned long long)V;
+  const int lz = __clzll((long long)m);
+  m <<= lz;
+  const int be = 1023 + 63 - lz + e;
+  if (be < 1) return 0.0;
+  if (be > 2045) return V < 0 ? -__longlong_as_double(0x7ff0000000000000ll) : __longlong_as_double(0x7ff0000000000000ll);
+  const unsigned long long q = (m >> 11) + ((m >> 10) & 1ull);
+  return __longlong_as_double((long long)((((unsigned long long)(be - 1)) << 52) + q + (V < 0 ? 1ull << 63 : 0ull)));
+}
+
+// Commit mode adds the samples to fdata; flux mode (a flux read with samples
+// still in the ring) leaves fdata as it is and forms the products of the four
+// flux components of 32 locations of one face, rows as in dft_ws: row 32 q +
+// 4 l + c is component c of location 8 q + l; one partial per (frequency,
+// tile, quarter), which k_flux_sum adds.
+template <bool FLUX> __global__ void __launch_bounds__(D64_THREADS, 1) k_dft_d64(D64Args A) {
+  extern __shared__ __align__(1024) unsigned char smem[];
+  unsigned short* sa = (unsigned short*)smem;   // [digit][D64_A]
+  unsigned short* sb = sa + D64_D * D64_A;      // [digit][D64_B]
+  __shared__ uint64_t bar_b, bar_a;
+  __shared__ uint32_t taddr_s;
+  __shared__ int stop_s, ex_s[D64_M];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const long i0 = A.nitems * blockIdx.x / gridDim.x, i1 = A.nitems * (blockIdx.x + 1) / gridDim.x;
+  if (tid == 0) {
+    mbar_init(&bar_b, 1);
+    mbar_init(&bar_a, 1);
+    stop_s = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&taddr_s)), "r"(512)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = taddr_s;
+  const long nsteps = (i1 - i0) * A.nsb;  // (item, sub-block) pairs
+  auto load_b = [&](long q) {             // thread 0: B of pair q
+    const long item = i0 + q / A.nsb, k = q % A.nsb;
+    mbar_expect_tx(&bar_b, 2u * D64_D * D64_B);
+    bulk_g2s(sb, A.Bt + (k * A.ngroups + item % A.ngroups) * (long)(D64_D * D64_B), 2u * D64_D * D64_B, &bar_b);
+  };
+  if (tid == 0 && nsteps > 0) load_b(0);
+  long have = -1;  // (tile, sub-block) whose digits are in A
+  bool go = true;
+  for (long item = i0; item < i1 && go; ++item) {
+    int g;
+    const WsRow<FLUX> wr = ws_item<FLUX>(A, item, g);
+    // epilogue: warp w reads lanes 32 (w % 4), columns 16 (w / 4) .. + 15
+    const int row = 32 * (warp & 3) + lane, c0 = 16 * (warp >> 2);
+    const int w0 = g * D64_F + c0 / 2;  // first of the warp's 8 frequencies
+    long p = ws_point<FLUX>(wr, row);
+    if (!bc_ok(p < A.P, BC_DFT_POINT, p)) p = -1;
+    double2 val[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      val[j] = p >= 0 && !A.fd_zero && w0 + j < A.nof ? A.fd[(long)(w0 + j) * A.P + p] : make_double2(0.0, 0.0);
+    for (int kb = 0; kb < A.nsb && go; ++kb) {
+      const long q = (item - i0) * A.nsb + kb;
+      const unsigned par = (unsigned)(q & 1);
+      const int nk = min(D64_S, A.nk - kb * D64_S);
+      if ((long)wr.tile * A.nsb + kb != have) {
+        // the digits of a tile's sub-block: thread = row and 8 samples (two
+        // runs of 4, 16 bytes of every digit plane each)
+        have = (long)wr.tile * A.nsb + kb;
+        const int r = tid & (D64_M - 1), h8 = tid >> 7;
+        long pr = ws_point<FLUX>(wr, r);
+        if (!bc_ok(pr < A.P, BC_DFT_SAMPLE, pr)) pr = -1;
+        double2 f[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+          f[k] = pr >= 0 && 8 * h8 + k < nk ? A.S[(long)(kb * D64_S + 8 * h8 + k) * A.P + pr] : make_double2(0.0, 0.0);
+        if (tid < D64_M) ex_s[tid] = 1;
+        __syncthreads();
+        int ex = 1;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          ex = max(ex, (int)((unsigned long long)__double_as_longlong(f[k].x) >> 52) & 0x7ff);
+          ex = max(ex, (int)((unsigned long long)__double_as_longlong(f[k].y) >> 52) & 0x7ff);
+        }
+        if (ex > 1) atomicMax(&ex_s[r], ex);
+        __syncthreads();
+        ex = ex_s[r];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          unsigned d[D64_D][4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            unsigned dr[D64_D], di[D64_D];
+            d64_digits(d64_int(f[4 * h + k].x, ex), dr);
+            d64_digits(d64_int(f[4 * h + k].y, ex), di);
+#pragma unroll
+            for (int s = 0; s < D64_D; ++s) d[s][k] = dr[s] | (di[s] << 16);
+          }
+#pragma unroll
+          for (int s = 0; s < D64_D; ++s)
+            *(uint4*)(sa + s * D64_A + d64_off(r, 16 * h8 + 8 * h)) = make_uint4(d[s][0], d[s][1], d[s][2], d[s][3]);
+        }
+        fence_proxy_async();  // the generic-proxy writes of A before the tensor core reads them
+        __syncthreads();
+      }
+      if (tid == 0) {
+        if (mbar_wait(&bar_b, par, STREAM_WAIT_CYCLES)) {
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const int nks = (2 * nk + 15) / 16;
+#pragma unroll 1
+          for (int o = 0; o < D64_O; ++o)
+#pragma unroll 1
+            for (int s = max(0, o - D64_D + 1); s <= min(o, D64_D - 1); ++s) {
+              const uint64_t da_ = d64_desc(sa + s * D64_A), db_ = d64_desc(sb + (o - s) * D64_B);
+              // 16 columns are two core matrices: 256 bytes, 16 in the descriptor's units
+              for (int ks = 0; ks < nks; ++ks)
+                d64_mma(tmem + (uint32_t)(o * D64_N), da_ + 16u * ks, db_ + 16u * ks,
+                        (s > max(0, o - D64_D + 1) || ks > 0) ? 1 : 0);
+            }
+          tc_commit(&bar_a);
+        } else {
+          atomicExch(A.err, FLUX ? 5 : 3);
+          *(volatile int*)&stop_s = 1;
+        }
+      }
+      __syncthreads();
+      if (*(volatile int*)&stop_s == 0 && !mbar_wait(&bar_a, par, STREAM_WAIT_CYCLES)) {
+        atomicExch(A.err, FLUX ? 5 : 3);
+        *(volatile int*)&stop_s = 1;
+      }
+      __syncthreads();
+      go = *(volatile int*)&stop_s == 0;
+      if (!go) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      if (tid == 0 && q + 1 < nsteps) load_b(q + 1);  // the MMAs have read this pair's B
+      const int ex = ex_s[row];
+      // the sum is V 2^(e' + eb' - 56), e' = ex - 1022, eb' = eb - 1022, V
+      // (below) at most 64 x 2^14 x 2^42 and rounded from 14 bits more
+      const int e2 = ex - 1022 + A.eb - 1022 - 56;
+#pragma unroll
+      for (int hf = 0; hf < 2; ++hf) {
+        long long hi[8], lo[8];
+#pragma unroll
+        for (int o = 0; o < D64_O; ++o) {
+          uint32_t t[8];
+          const uint32_t ta = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(o * D64_N + c0 + 8 * hf);
+          asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+                       : "=r"(t[0]), "=r"(t[1]), "=r"(t[2]), "=r"(t[3]), "=r"(t[4]), "=r"(t[5]), "=r"(t[6]), "=r"(t[7])
+                       : "r"(ta)
+                       : "memory");
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            const long long v = (long long)__float2int_rn(__uint_as_float(t[c]));
+            if (o == 0) hi[c] = v;
+            else if (o < 4) hi[c] = hi[c] * 256 + v;
+            else if (o == 4) lo[c] = v;
+            else lo[c] = lo[c] * 256 + v;
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          double2& v = val[4 * hf + j];
+          if (ex == 0x7ff) {
+            v.x = v.y = __longlong_as_double(0x7ff8000000000000ll);
+          } else {
+            v.x = da(v.x, d64_value(hi[2 * j] * 262144 + ((lo[2 * j] + 8192) >> 14), e2));
+            v.y = da(v.y, d64_value(hi[2 * j + 1] * 262144 + ((lo[2 * j + 1] + 8192) >> 14), e2));
+          }
+        }
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncthreads();  // every lane has read the accumulators before the next MMAs
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    }
+    if (!go) break;
+    if (FLUX) {
+#pragma unroll 1
+      for (int j = 0; j < 8; ++j) {
+        // lanes c = 0 and c = 2: Re(a conj b) and -Re(c conj d), then the sum
+        // of the 8 locations' lanes in a fixed tree
+        double2 v = val[0];
+#pragma unroll
+        for (int t = 1; t < 8; ++t)
+          if (t == j) v = val[t];
+        const double bx = __shfl_xor_sync(0xffffffffu, v.x, 1), by = __shfl_xor_sync(0xffffffffu, v.y, 1);
+        double s = fma(v.y, by, dm(v.x, bx));
+        if (lane & 2) s = -s;
+#pragma unroll
+        for (int m = 2; m < 32; m <<= 1) s = da(s, __shfl_xor_sync(0xffffffffu, s, m));
+        if (lane == 0 && w0 + j < A.nof)
+          A.part[(long)(w0 + j) * (4L * A.ft.start[6]) + 4L * wr.tile + (warp & 3)] = s;
+      }
+    } else if (p >= 0) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (w0 + j < A.nof) A.fd[(long)(w0 + j) * A.P + p] = val[j];
+    }
+  }
+  // a copy still in flight lands before the CTA exits
+  if (tid == 0 && !go) mbar_wait(&bar_b, 0, STREAM_WAIT_CYCLES >> 4);
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 0)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+}
 
 // J[f][iw] = scale * sign * (sum of face f's partials, four per tile, in
 // order within each thread, then a fixed tree).
@@ -2586,18 +2875,37 @@ int build_dft(iris_engine* E) {
 
 namespace iris {
 
+// The FP64 block kernel's arguments for the first nk samples of the ring, its
+// twiddle operands launched.
+static D64Args d64_args(iris_engine* E, int nk) {
+  D64Args A{};
+  A.S = (const double2*)E->S;
+  A.P = E->P;
+  A.nk = nk;
+  A.nsb = (nk + D64_S - 1) / D64_S;
+  A.Bt = (const __nv_bfloat16_raw*)E->d_wt64;
+  A.fd = (double2*)E->fd;
+  A.fd_zero = E->fd_zero;
+  A.nof = E->p.nof;
+  A.ngroups = (E->p.nof + D64_F - 1) / D64_F;
+  A.eb = std::ilogb(E->p.dt) + 1023;
+  A.err = E->d_err;
+  k_twiddle_d64<<<(unsigned)(A.nsb * A.ngroups * D64_F * D64_S / 256), 256, 0, E->st>>>(
+      E->d_tk, nk, E->d_fw, A.nof, E->p.dt, A.ngroups, (__nv_bfloat16_raw*)E->d_wt64);
+  return A;
+}
+
 void dft_flush(iris_engine* E) {
   if (E->nslot == 0) return;
   KTimer tm(E, IRIS_KC_DFT);
   const int nk = E->nslot;
   // the CUDA-core blocks read what they add to (on a failure the samples stay buffered)
-  if (!E->dft_tc && fd_materialise(E)) return;
+  if (E->prec != IRIS_FP64 && !E->dft_tc && fd_materialise(E)) return;
   if (E->prec == IRIS_FP64) {
-    const int nwc = (E->p.nof + DFT64_WC - 1) / DFT64_WC;
-    const long nblk = (E->P + 127) / 128;
-    k_twiddle64<<<(nk * E->p.nof + 255) / 256, 256, 0, E->st>>>(E->d_tk, nk, E->d_fw, E->p.nof, E->d_wt64);
-    k_dft_fp64<<<(unsigned)(nblk * nwc), 128, (size_t)nk * DFT64_WC * sizeof(double2), E->st>>>(
-        (const double2*)E->S, E->P, nk, E->d_wt64, E->p.nof, nwc, E->p.dt, (double2*)E->fd);
+    D64Args A = d64_args(E, nk);
+    A.nitems = (E->P + D64_M - 1) / D64_M * A.ngroups;
+    k_dft_d64<false><<<(unsigned)std::min<long>(A.nitems, E->ws_blocks), D64_THREADS, D64_SMEM, E->st>>>(A);
+    E->fd_zero = false;  // every accumulator of every frequency has been written
   } else if (E->dft_tc) {
     const int ng = (E->p.nof + TC_NW - 1) / TC_NW, nch = (2 * nk + TC_KC - 1) / TC_KC;
     const long nt = (long)ng * nch * TC_BROWS * TC_KC;
@@ -2689,8 +2997,7 @@ int alloc_dft(iris_engine* E, const FluxFace* faces, int nfaces) {
   CK(cudaMemGetInfo(&freeb, &totb));
   const size_t fd_bytes = (size_t)P * p.nof * sizeof(double2);
   if (fd_bytes > freeb) return fail(IRIS_ENOMEM, "DFT accumulators exceed free device memory");
-  // FP64: at most 256 slots (its block kernel stages K x 8 twiddles in 32 KB
-  // of shared memory), 32 by default.  FP32: up to 512, the default: a block
+  // FP64: at most 256 slots, 32 by default (accumulated 32 at a time).  FP32: up to 512, the default: a block
   // reads and writes the FP64 accumulators once, so a longer block moves
   // fewer accumulator bytes per sample.  The ring takes at most half of the
   // memory left after the accumulators.
@@ -2708,17 +3015,23 @@ int alloc_dft(iris_engine* E, const FluxFace* faces, int nfaces) {
   CK(cudaMalloc(&E->d_fw, sizeof(double) * p.nof));
   CK(cudaMemcpy(E->d_fw, E->fw.data(), sizeof(double) * p.nof, cudaMemcpyHostToDevice));
   if (E->prec == IRIS_FP32) CK(cudaMalloc(&E->d_wt, sizeof(float2) * (size_t)E->K * p.nof));
-  if (E->prec == IRIS_FP64) CK(cudaMalloc(&E->d_wt64, sizeof(double2) * (size_t)E->K * p.nof));
+  if (E->prec == IRIS_FP64) {
+    CK(cudaMalloc(&E->d_wt64, 2 * (size_t)D64_D * D64_B * ((p.nof + D64_F - 1) / D64_F) * ((E->K + D64_S - 1) / D64_S)));
+    CK(cudaFuncSetAttribute(k_dft_d64<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)D64_SMEM));
+    CK(cudaFuncSetAttribute(k_dft_d64<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)D64_SMEM));
+  }
   E->dft_tc = E->prec == IRIS_FP32 && p.dft_kernel != IRIS_DFT_KERNEL_CUDA;
   E->flux_faces.assign(faces, faces + nfaces);
+  int nsm = 0;
+  CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, E->device));
+  E->ws_blocks = std::max(1, nsm);  // one persistent CTA per SM (its TMEM takes all 512 columns)
   if (E->dft_tc) {
     const int ng = (p.nof + TC_NW - 1) / TC_NW, nch = (2 * E->K + TC_KC - 1) / TC_KC;
     CK(cudaMalloc(&E->d_wtc, sizeof(float) * (size_t)ng * nch * 2 * TC_BROWS * TC_KC));
     CK(cudaFuncSetAttribute(k_dft_ws_commit, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WS_SMEM));
     CK(cudaFuncSetAttribute(k_dft_ws_flux, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WS_SMEM));
-    int nsm = 0;
-    CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, E->device));
-    E->ws_blocks = std::max(1, nsm);  // one persistent CTA per SM (its TMEM takes all 512 columns)
+  }
+  if (E->dft_tc || E->prec == IRIS_FP64) {
     long maxt = 1;
     for (int s = 0; s + 6 <= nfaces; s += 6) maxt = std::max(maxt, (long)flux_tiles(faces + s).start[6]);
     CK(cudaMalloc(&E->d_part, sizeof(double) * 4 * (size_t)maxt * p.nof));
@@ -2730,6 +3043,10 @@ int alloc_dft(iris_engine* E, const FluxFace* faces, int nfaces) {
   CK(cudaMalloc(&E->d_faces, sizeof(FluxFace) * nfaces));
   CK(cudaMemcpy(E->d_faces, faces, sizeof(FluxFace) * nfaces, cudaMemcpyHostToDevice));
   CK(cudaMalloc(&E->d_J, sizeof(double) * 6 * p.nof));
+  if (!E->d_err) {  // a batch's shell: the tensor-core blocks record a wait that gave up
+    CK(cudaMalloc(&E->d_err, sizeof(int)));
+    CK(cudaMemset(E->d_err, 0, sizeof(int)));
+  }
   CK(cudaMallocHost(&E->h_J, sizeof(double) * 6 * p.nof));
   return IRIS_OK;
 }
@@ -2995,10 +3312,12 @@ static int stream_status(iris_engine* E) {
   return fail(IRIS_ETIMEOUT, what);
 }
 
-// The flux of one face set.  FP32 mode on the tensor cores: over the
-// accumulators plus the samples still in the ring, which stay there
-// (k_twiddle_tc for the pending samples, k_dft_ws_flux, k_flux_sum).  Otherwise
-// the ring is committed first and k_flux reads the accumulators.
+// The flux of one face set.  On the tensor cores: over the accumulators plus
+// the samples still in the ring, which stay there (FP32: k_twiddle_tc for the
+// pending samples, k_dft_ws_flux, k_flux_sum; FP64: k_twiddle_d64, k_dft_d64,
+// k_flux_sum, or k_flux when none are pending).  A flux read so never splits a
+// block of samples, whose sums round per block.  On the CUDA cores the ring is
+// committed first and k_flux reads the accumulators.
 int iris::read_flux(iris_engine* E, int set, double* J) {
   const iris_params& p = E->p;
   const double scale = p.eps0 * p.Q / (2.0 * p.dt);
@@ -3030,6 +3349,17 @@ int iris::read_flux(iris_engine* E, int set, double* J) {
       A.part = E->d_part;
       A.err = E->d_err;
       k_dft_ws_flux<<<(unsigned)std::min<long>(A.nitems, E->ws_blocks), WsCfg<true>::THREADS, WS_SMEM, E->st>>>(A);
+    }
+    k_flux_sum<<<dim3(p.nof, 6), 256, 0, E->st>>>(E->d_part, ft, E->d_faces + 6 * set, p.nof, scale, E->d_J);
+  } else if (E->prec == IRIS_FP64 && E->nslot > 0) {
+    KTimer tm(E, IRIS_KC_FLUX);
+    if (ft.start[6] > 0) {
+      D64Args A = d64_args(E, E->nslot);
+      A.nitems = (long)ft.start[6] * A.ngroups;
+      A.faces = E->d_faces + 6 * set;
+      A.ft = ft;
+      A.part = E->d_part;
+      k_dft_d64<true><<<(unsigned)std::min<long>(A.nitems, E->ws_blocks), D64_THREADS, D64_SMEM, E->st>>>(A);
     }
     k_flux_sum<<<dim3(p.nof, 6), 256, 0, E->st>>>(E->d_part, ft, E->d_faces + 6 * set, p.nof, scale, E->d_J);
   } else {

@@ -79,7 +79,7 @@ struct iris_engine {
   // (fd_materialise)
   bool fd_zero = false;
   float2* d_wt = nullptr;
-  double2* d_wt64 = nullptr;  // FP64 mode twiddles of one block
+  void* d_wt64 = nullptr;  // FP64 mode: B operands of 32 samples (k_twiddle_d64)
   bool dft_tc = false;     // FP32 block accumulation on the tensor cores
   float* d_wtc = nullptr;  // its B operands (k_twiddle_tc)
   int ws_blocks = 0;       // CTAs of its persistent launches (one per SM)
