@@ -37,6 +37,7 @@
 
 #include "iris_engine.h"
 #include "iris_fused.cuh"
+#include "iris_march.cuh"
 
 namespace iris {
 namespace {
@@ -92,39 +93,13 @@ constexpr size_t STREAM_SMEM_E = SNST * sizeof(StageE);
 constexpr size_t STREAM_SMEM_H = SNST * sizeof(StageH);
 
 
-__device__ __forceinline__ void mbar_init(uint64_t* bar, unsigned count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, unsigned bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, unsigned parity) {
-  unsigned ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// Waits for phase parity of bar for at most about limit clock cycles;
-// false when it gave up.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity, long long limit) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const long long t0 = clock64();
-  while (!mbar_try_wait(bar, parity))
-    if (clock64() - t0 > limit) return false;
-  return true;
-}
 __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, unsigned bytes, uint64_t* bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
                    smem_u32(dst)),
                "l"(src), "r"(bytes), "r"(smem_u32(bar))
                : "memory");
 }
-__device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
-constexpr long long STREAM_WAIT_CYCLES = 1LL << 31;  // about a second
 
 // IRIS_OP_WAIT_CHECK: an mbarrier armed for 16 bytes that no copy delivers,
 // waited on with the streamed passes' limit divided by 2^shift; the give-up
@@ -2003,6 +1978,21 @@ __global__ void __launch_bounds__(FZ_X* FZ_Y, 2) k_fused(FusedArgs A) {
   fused_column<CEPS, UPML, IT>(A, S, U, blockIdx.x, blockIdx.y, z0, z1);
 }
 
+// The planes outside the UPML slabs by staged tiles (iris_march.cuh).
+template <typename TL, bool CEPS> __global__ void __launch_bounds__(MR_T, 2) k_march(MarchArgs A) {
+  extern __shared__ __align__(128) unsigned char mr_dyn[];
+  const int z0 = A.za + A.zc * (int)blockIdx.z, z1 = min(z0 + A.zc - 1, A.zb);
+  march_tile<TL, CEPS>(A, mr_dyn, blockIdx.x, blockIdx.y, z0, z1);
+}
+using MarchFn = void (*)(MarchArgs);
+MarchFn march_kernel(int id, bool cplx) {
+#define IRIS_MARCH_K(ID, W, R) \
+  if (id == ID) return cplx ? (MarchFn)k_march<MarchTile<W, R>, true> : (MarchFn)k_march<MarchTile<W, R>, false>;
+  IRIS_MARCH_SHAPES(IRIS_MARCH_K)
+#undef IRIS_MARCH_K
+  return nullptr;
+}
+
 }  // namespace
 
 // ---------------------------------------------------------------------------
@@ -2227,22 +2217,42 @@ double fused_fill(int nx, int ny) {
   return (double)nx * ny / ((double)tx * FZ_X * ty * FZ_Y);
 }
 
-// z chunks of planes za..zb for a launch over `tiles` column tiles: about
-// 32 waves of two CTAs per SM, at least 48 planes each (each chunk also
-// reads the H plane below it and forms E' on the plane above it; measured
-// on GB300 against 8 waves of at least 16
-// planes: 512x512x1024 4.91 against 5.04 ms a pass, 160x160x512 0.378
-// against 0.389, 512x512x256 and 256x256x512 the same); appends (za, zb,
-// planes per chunk, chunks) to r.
+// z chunks of planes za..zb for a launch of fused_column over `tiles` column
+// tiles: at least 48 planes each where the tiles fill the chip (each chunk
+// also reads the H plane below it and forms E' on the plane above it; measured
+// on GB300 against 16 planes: 512x512x1024 4.91 against 5.04 ms a pass), and
+// as few as 4 where they do not: a slab of 17 planes in one chunk is a chain
+// of 17 planes' latencies (64x64x512: 118 us a step, with 5 planes 90;
+// 128x128x128 111 and 87).
+// Appends (za, zb, planes per chunk, chunks) to r.
 void fused_chunks(std::vector<int>& r, int za, int zb, long tiles) {
   if (zb < za) return;
   const int len = zb - za + 1;
-  long nch = std::max(1L, (32L * 152 * 2 + tiles - 1) / tiles);
-  nch = std::min<long>(nch, std::max(1, len / 48));
+  const long full = 2 * 152;
+  long nch = std::min<long>((32 * full + tiles - 1) / tiles, std::max(1, len / 48));
+  nch = std::max(nch, std::min<long>((full / 2 + tiles - 1) / tiles, len / 4));
   const int zc = (int)((len + nch - 1) / nch);
   r.insert(r.end(), {za, zb, zc, (len + zc - 1) / zc});
 }
 
+// The march of planes (za, zb, zc, n) on the engine's stream.
+void launch_march(iris_engine* E, const std::vector<int>& r) {
+  MarchArgs a{};
+  a.f = field_args<float>(E);
+  a.e_new = (float2*)E->e2;
+  a.h_new = (float2*)E->h2;
+  a.tx = E->mshape.tx;
+  a.ty = E->mshape.ty;
+  a.za = r[0], a.zb = r[1], a.zc = r[2];
+  march_kernel(E->mshape.id, E->eps_complex)<<<dim3(a.tx, a.ty, r[3]), MR_T, E->mshape.smem, E->st>>>(a);
+}
+
+// z chunks of the march: MR_CHUNK to 2 MR_CHUNK - 1 planes each.  Appends
+// (za, zb, planes per chunk, chunks) to r.
+void march_chunks(std::vector<int>& r, int za, int zb) {
+  const int len = zb - za + 1, n = std::max(1, len / MR_CHUNK), zc = (len + n - 1) / n;
+  r.insert(r.end(), {za, zb, zc, (len + zc - 1) / zc});
+}
 
 // One fused step into the second buffers, swap, then TF/SF and the DFT
 // sample on the new state, in the operator order of the split passes; step
@@ -2260,19 +2270,18 @@ void fused_one(iris_engine* E, int it, int left, const int* itp, bool sampled) {
       cudaEventRecord(E->fz_fork, E->st);
       cudaStreamWaitEvent(E->st2, E->fz_fork, 0);
     }
-    for (int part = 0; part < 2; ++part) {
+    for (int part = 1; part >= 0; --part) {
       const std::vector<int>& r = E->fzr[part];
       if (r.empty()) continue;
+      if (part == 0 && E->mshape.id >= 0) {
+        launch_march(E, r);
+        continue;
+      }
       const FusedArgs a = fused_args(E, part);
       const dim3 grd(E->fgrd.x, E->fgrd.y, (unsigned)(r[3] + (r.size() > 4 ? r[7] : 0)));
       if (part == 0) {
-        if (E->fz_i32) {
-          if (E->eps_complex) k_fused<true, false, int><<<grd, E->fblk, 0, E->st>>>(a);
-          else k_fused<false, false, int><<<grd, E->fblk, 0, E->st>>>(a);
-        } else {
-          if (E->eps_complex) k_fused<true, false, long><<<grd, E->fblk, 0, E->st>>>(a);
-          else k_fused<false, false, long><<<grd, E->fblk, 0, E->st>>>(a);
-        }
+        if (E->eps_complex) k_fused<true, false, long><<<grd, E->fblk, 0, E->st>>>(a);
+        else k_fused<false, false, long><<<grd, E->fblk, 0, E->st>>>(a);
       } else {
         cudaStream_t s = both ? E->st2 : E->st;
         if (E->fz_i32) {
@@ -3246,14 +3255,26 @@ int create_engine(const iris_params* pin, const double* fw, bool member, bool z_
     const int ia = p.pmlzi + 1, ib = p.pmlzf - 2;
     for (int part = 0; part < 2; ++part) E->fzr[part].clear();
     if (ib >= ia) {
-      fused_chunks(E->fzr[0], ia, ib, tiles);
+      // the staged march where its tiles fill and 32-bit offsets reach
+      if (3 * g.comp < (1L << 31)) {
+        E->mshape = march_shape(p.nx, p.ny);
+        march_chunks(E->fzr[0], ia, ib);
+        for (bool c : {false, true})
+          if (cudaFuncSetAttribute((const void*)march_kernel(E->mshape.id, c), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)E->mshape.smem) != cudaSuccess)
+            return bail(fail(IRIS_ECUDA, "fused pass: shared memory configuration failed"));
+      } else {
+        fused_chunks(E->fzr[0], ia, ib, tiles);
+      }
       fused_chunks(E->fzr[1], 1, ia - 1, tiles);
       fused_chunks(E->fzr[1], ib + 1, p.nz, tiles);
     } else {
       fused_chunks(E->fzr[1], 1, p.nz, tiles);
     }
     E->fblk = dim3(FZ_X, FZ_Y, 1);
-    if (cudaStreamCreateWithFlags(&E->st2, cudaStreamNonBlocking) != cudaSuccess ||
+    int prio_lo = 0, prio_hi = 0;
+    cudaDeviceGetStreamPriorityRange(&prio_lo, &prio_hi);
+    if (cudaStreamCreateWithPriority(&E->st2, cudaStreamNonBlocking, prio_hi) != cudaSuccess ||
         cudaEventCreateWithFlags(&E->fz_fork, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&E->fz_join, cudaEventDisableTiming) != cudaSuccess)
       return bail(fail(IRIS_ECUDA, "fused pass: stream creation failed"));

@@ -14,6 +14,7 @@
 
 #include "iris_device.cuh"
 #include "iris_internal.h"
+#include "iris_march.cuh"
 #include "iris_resident.cuh"
 
 // Return IRIS_ECUDA (IRIS_ENOMEM for an allocation) with the failing call's
@@ -103,6 +104,7 @@ struct iris_engine {
   // the UPML slabs, [1] the slabs
   std::vector<int> fzr[2];
   dim3 fblk, fgrd;
+  iris::MarchShape mshape;  // tile shape of the staged pass of [0] (id < 0: not used)
   bool fz_i32 = false;  // the fused pass's offsets fit int (3 x comp < 2^31)
   // the slab launch runs on st2, concurrently with the interior launch (they
   // write disjoint planes and read only the old state): fork / join events

@@ -21,7 +21,7 @@ LIB = LIB_BC if os.environ.get("IRIS_BOUNDS_CHECK") == "1" else LIB_PLAIN
 SOURCES = ["iris_engine.cu", "iris_batch.cu", "iris_adjoint.cu", "iris_host.cpp"]
 HEADERS = [os.path.join(INCLUDE, "iris_fdtd.h")] + [os.path.join(CSRC, h) for h in
                                                    ("iris_internal.h", "iris_device.cuh", "iris_engine.h",
-                                                    "iris_fused.cuh", "iris_resident.cuh")]
+                                                    "iris_fused.cuh", "iris_march.cuh", "iris_resident.cuh")]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 
 
