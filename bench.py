@@ -516,7 +516,7 @@ def measure_batch(iris, args, rank, world, local, K, W, D, loop_sample=0):
         eb += e
         hb += h
     if kn["fused_eh"] > 0:
-        # the fused work list: one pass per step (its launches each timed) moves both passes' bytes
+        # the fused work list: one pass per step (one timer over its launches) moves both passes' bytes
         t_f = kms["fused_eh"] / K * 1e-3
         dom, db, dt_ = "fused_eh", eb + hb, t_f
         t_e = t_h = t_f / 2
@@ -526,7 +526,7 @@ def measure_batch(iris, args, rank, world, local, K, W, D, loop_sample=0):
         dom, db, dt_ = ("update_h", hb, t_h) if t_h >= t_e else ("update_e", eb, t_e)
     achieved = db / dt_ / 1e9
     flux_launches = 3 if buffered else 2
-    launches = info["launches_per_pass"] * (kn["update_e"] + kn["update_h"]) + kn["fused_eh"] + \
+    launches = info["launches_per_pass"] * (kn["update_e"] + kn["update_h"] + kn["fused_eh"]) + \
         kn["tfsf"] + kn["dft_gather"] + kn["flux"] * flux_launches + 2 * kn["dft_block"]
     value = world * cells * K / (reg_ms * 1e-3) / 1e9
     h2d = 0  # the patterns are generated on the device

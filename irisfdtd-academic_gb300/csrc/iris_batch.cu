@@ -48,7 +48,8 @@ struct BSeg {
   int cell, pad;
 };
 struct FItem {
-  int cell, bx, by, z0, z1, pad;  // column tile (bx, by) of cell, planes z0..z1
+  int cell, bx, by, z0, z1;  // column tile (bx, by) of cell, planes z0..z1
+  int pad;
 };
 
 // Work-list shapes the autotuner chooses from: x * y * z blocks of cells,
@@ -175,6 +176,40 @@ __global__ void __launch_bounds__(FZ_X* FZ_Y, 2) k_batch_fused(const FusedArgs* 
   }
 }
 
+// The same for the planes outside the slabs by staged tiles (iris_march.cuh):
+// blockIdx.y is the cell, blockIdx.x its (x tile, y tile, z chunk); CTAs past
+// the cell's last leave at once.  The cells' arguments are kernel parameters,
+// MARCH_CELLS a launch, indexed by blockIdx alone: they are then read through
+// the uniform datapath.  Copied to shared memory instead they were read from
+// there, or held in registers, in every plane: 4.44 ms against 4.20 for 32
+// ragged cells of 182 million points, whose E and H passes over flat runs take
+// 5.26; their 96 bytes a point take 2.6 at the measured copy bandwidth.  The
+// UPML slabs (k_batch_fused) and the tiles' unfilled threads (a fifth) make
+// up most of the difference.
+constexpr int MARCH_CELLS = 48;
+struct MarchCell {
+  MarchArgs a;
+  int za, zb, zc, n;  // planes za..zb, zc a chunk; CTAs
+  int shape;
+};
+struct MarchCells {
+  MarchCell c[MARCH_CELLS];
+};
+template <bool CEPS> __global__ void __launch_bounds__(MR_T, 2) k_batch_march(const __grid_constant__ MarchCells P) {
+  extern __shared__ __align__(128) unsigned char mr_dyn[];
+  const MarchCell& c = P.c[blockIdx.y];
+  if ((int)blockIdx.x >= c.n) return;
+  const int tiles = c.a.tx * c.a.ty, iz = blockIdx.x / tiles, t = blockIdx.x - iz * tiles;
+  const int by = t / c.a.tx, bx = t - by * c.a.tx, z0 = c.za + iz * c.zc, z1 = min(z0 + c.zc - 1, c.zb);
+#define IRIS_MARCH_CASE(ID, W, R)                                                              \
+  case ID:                                                                                     \
+    if (CEPS && c.a.f.eps_c) march_tile<MarchTile<W, R>, true>(c.a, mr_dyn, bx, by, z0, z1);    \
+    else march_tile<MarchTile<W, R>, false>(c.a, mr_dyn, bx, by, z0, z1);                      \
+    break;
+  switch (c.shape) { IRIS_MARCH_SHAPES(IRIS_MARCH_CASE) }
+#undef IRIS_MARCH_CASE
+}
+
 // The TF/SF corrections of steps it0 .. it0+n-1 (from *itp on when given) for
 // every column of every cell: column q of a table row is column cols[q].y of
 // cell cols[q].x.
@@ -237,6 +272,13 @@ struct iris_batch {
   bool second = false;
   int parity = 0;
   void* d_fargs = nullptr;
+  // the planes outside the slabs of the cells that march (all but those too
+  // large for its 32-bit offsets, which have FUSED items), per parity; the
+  // slab launch runs on st2, as in the single engine
+  std::vector<MarchCell> march[2];
+  size_t march_smem = 0;
+  cudaStream_t st2 = nullptr;
+  cudaEvent_t fork = nullptr, join = nullptr;
   FItem* d_fitems = nullptr;
   SrcArgs* d_src = nullptr;
   BItem* d_items = nullptr;
@@ -264,6 +306,27 @@ void swap_sets(iris_engine* E) {
   std::swap(E->e, E->e2);
   std::swap(E->h, E->h2);
   for (int s = 0; s < 2; ++s) std::swap(E->pml_d[s], E->pml_d2[s]);
+}
+
+// The march's cells (second buffers present), for both buffer parities.
+void batch_march_cells(iris_batch* B) {
+  B->march_smem = 0;
+  for (int q = 0; q < 2; ++q) {
+    B->march[q].clear();
+    for (iris_engine* E : B->cells) {
+      const int ia = E->p.pmlzi + 1, ib = E->p.pmlzf - 2;
+      if (ib < ia || E->mshape.id < 0) continue;
+      if (q != B->parity) swap_sets(E);
+      MarchCell m{};
+      m.a = march_args(E);
+      if (q != B->parity) swap_sets(E);
+      m.za = ia, m.zb = ib, m.zc = march_chunk(ib - ia + 1);
+      m.n = m.a.tx * m.a.ty * ((ib - ia + m.zc) / m.zc);
+      m.shape = E->mshape.id;
+      B->march[q].push_back(m);
+      B->march_smem = std::max(B->march_smem, E->mshape.smem);
+    }
+  }
 }
 
 // The cells' kernel arguments for both buffer parities.  A member's own
@@ -299,6 +362,8 @@ int batch_upload_args(iris_batch* B) {
   if (B->second) {
     if (!B->d_fargs) CK(cudaMalloc(&B->d_fargs, sizeof(FusedArgs) * fa.size()));
     CK(cudaMemcpy(B->d_fargs, fa.data(), sizeof(FusedArgs) * fa.size(), cudaMemcpyHostToDevice));
+    batch_march_cells(B);
+    graph_reset(B->master);  // captured march launches hold the cells' arguments
   }
   return IRIS_OK;
 }
@@ -329,7 +394,15 @@ int batch_drop_second(iris_batch* B) {
 // The members' second field buffers and D (zero), for the FUSED work list.
 int batch_second_buffers(iris_batch* B) {
   if (B->second) return IRIS_OK;
+  if (!B->st2) {
+    int lo = 0, hi = 0;
+    CK(cudaDeviceGetStreamPriorityRange(&lo, &hi));
+    CK(cudaStreamCreateWithPriority(&B->st2, cudaStreamNonBlocking, hi));
+    CK(cudaEventCreateWithFlags(&B->fork, cudaEventDisableTiming));
+    CK(cudaEventCreateWithFlags(&B->join, cudaEventDisableTiming));
+  }
   for (iris_engine* E : B->cells) {
+    if (3 * E->g.comp < (1L << 31)) E->mshape = march_shape(E->p.nx, E->p.ny);
     const size_t fbytes = (size_t)3 * E->g.comp * E->esz;
     if (!E->e2) CK(cudaMalloc(&E->e2, fbytes));
     if (!E->h2) CK(cudaMalloc(&E->h2, fbytes));
@@ -345,10 +418,10 @@ int batch_second_buffers(iris_batch* B) {
   return batch_upload_args(B);
 }
 
-// FUSED items: every cell's planes outside its UPML slabs in chunks of
-// FB_CHUNK (stopping at pmlzf-2, as the single-engine launch does) first,
-// then its two slabs each with the plane next to it; within a chunk, tile
-// rows of the cell in order.
+// FUSED items: the planes outside the UPML slabs (stopping at pmlzf-2, as the
+// single-engine launch does) of the cells that do not march, in chunks of
+// FB_CHUNK, then every cell's two slabs each with the plane next to it;
+// within a chunk, tile rows of the cell in order.
 int batch_build_fused_items(iris_batch* B) {
   std::vector<FItem> in, slab;
   for (int c = 0; c < B->n; ++c) {
@@ -361,7 +434,7 @@ int batch_build_fused_items(iris_batch* B) {
     };
     const int ia = p.pmlzi + 1, ib = p.pmlzf - 2;
     if (ib >= ia) {
-      add(in, ia, ib, FB_CHUNK);
+      if (B->cells[c]->mshape.id < 0) add(in, ia, ib, FB_CHUNK);
       add(slab, 1, ia - 1, p.nz);
       add(slab, ib + 1, p.nz, p.nz);
     } else {
@@ -372,6 +445,8 @@ int batch_build_fused_items(iris_batch* B) {
   in.insert(in.end(), slab.begin(), slab.end());
   for (const void* kf : {(const void*)k_batch_fused<false, true>, (const void*)k_batch_fused<true, true>})
     CK(cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FZ_UPML_SMEM));
+  for (const void* kf : {(const void*)k_batch_march<false>, (const void*)k_batch_march<true>})
+    CK(cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, MARCH_MAX_SMEM));
   graph_reset(B->master);
   if (B->d_fitems) cudaFree(B->d_fitems);
   B->d_fitems = nullptr;
@@ -485,25 +560,49 @@ template <typename T, int MINB> void launch_batch_flat(iris_batch* B, bool e) {
   else launch_flat<T, MINB, false>(B, e);
 }
 
-// One fused E+H pass of every cell (FUSED work list, FP32): the items
-// outside the slabs, then the slab items; the buffer sets then swap.
+// One fused E+H pass of every cell (FUSED work list, FP32): the slab items on
+// the second stream, the items outside the slabs, then the buffer sets swap.
 template <bool CEPS> void launch_batch_fused(iris_batch* B) {
   iris_engine* M = B->master;
-  const FusedArgs* args = (const FusedArgs*)B->d_fargs + (size_t)B->parity * B->n;
-  for (int part = 0; part < 2; ++part) {
-    const long n = part == 0 ? B->nitems_in : B->nitems - B->nitems_in;
-    if (n <= 0) continue;
-    const FItem* items = B->d_fitems + (part == 0 ? 0 : B->nitems_in);
-    const void* kern = part == 0 ? (const void*)k_batch_fused<CEPS, false> : (const void*)k_batch_fused<CEPS, true>;
-    const size_t dyn = part == 0 ? 0 : FZ_UPML_SMEM;
-    static int per[2] = {0, 0};
-    if (!per[part]) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[part], kern, FZ_X * FZ_Y, dyn);
-    int nsm = 0;
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, B->device);
-    const unsigned g = (unsigned)std::min<long>(n, (long)nsm * std::max(1, per[part]));
-    KTimer tm(M, IRIS_KC_FUSED);
-    if (part == 0) k_batch_fused<CEPS, false><<<g, dim3(FZ_X, FZ_Y), 0, M->st>>>(args, items, n);
-    else k_batch_fused<CEPS, true><<<g, dim3(FZ_X, FZ_Y), FZ_UPML_SMEM, M->st>>>(args, items, n);
+  const size_t set = (size_t)B->parity * B->n;
+  const FusedArgs* args = (const FusedArgs*)B->d_fargs + set;
+  const long nslab = B->nitems - B->nitems_in, nbig = B->nitems_in;
+  const std::vector<MarchCell>& mc = B->march[B->parity];
+  int nsm = 0;
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, B->device);
+  const dim3 blk(FZ_X, FZ_Y);
+  auto ctas = [&](const void* kern, size_t dyn, long n, int& per) {
+    if (!per) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, FZ_X * FZ_Y, dyn);
+    return (unsigned)std::min<long>(n, (long)nsm * std::max(1, per));
+  };
+  static int per_in = 0, per_slab = 0;
+  KTimer tm(M, IRIS_KC_FUSED);
+  const bool both = nslab > 0 && (nbig > 0 || !mc.empty());
+  if (both) {
+    cudaEventRecord(B->fork, M->st);
+    cudaStreamWaitEvent(B->st2, B->fork, 0);
+  }
+  if (nslab > 0) {
+    const unsigned g = ctas((const void*)k_batch_fused<CEPS, true>, FZ_UPML_SMEM, nslab, per_slab);
+    k_batch_fused<CEPS, true><<<g, blk, FZ_UPML_SMEM, both ? B->st2 : M->st>>>(args, B->d_fitems + B->nitems_in, nslab);
+  }
+  for (size_t i = 0; i < mc.size(); i += MARCH_CELLS) {
+    MarchCells P;
+    const size_t n = std::min<size_t>(MARCH_CELLS, mc.size() - i);
+    int ctas = 0;
+    for (size_t j = 0; j < n; ++j) {
+      P.c[j] = mc[i + j];
+      ctas = std::max(ctas, P.c[j].n);
+    }
+    k_batch_march<CEPS><<<dim3(ctas, (unsigned)n), MR_T, B->march_smem, M->st>>>(P);
+  }
+  if (nbig > 0) {
+    const unsigned g = ctas((const void*)k_batch_fused<CEPS, false>, 0, nbig, per_in);
+    k_batch_fused<CEPS, false><<<g, blk, 0, M->st>>>(args, B->d_fitems, nbig);
+  }
+  if (both) {
+    cudaEventRecord(B->join, B->st2);
+    cudaStreamWaitEvent(M->st, B->join, 0);
   }
   B->parity ^= 1;
   for (iris_engine* E : B->cells) swap_sets(E);
@@ -598,6 +697,9 @@ void batch_free(iris_batch* B) {
                   B->d_tcols, B->d_tfv};
   for (void* q : ptrs)
     if (q) cudaFree(q);
+  if (B->st2) cudaStreamDestroy(B->st2);
+  if (B->fork) cudaEventDestroy(B->fork);
+  if (B->join) cudaEventDestroy(B->join);
   if (B->master) {
     free_engine(B->master);
     delete B->master;
@@ -944,7 +1046,10 @@ int iris_batch_info(const iris_batch* B, long* info) {
   info[3] = B->master->K;
   info[4] = B->tile;
   info[5] = B->nitems;
-  info[6] = B->tile >= FLAT ? (B->nitems_in > 0) + (B->nitems > B->nitems_in) : 1;  // per E, H or fused pass
+  if (B->tile == FUSED)
+    for (const MarchCell& m : B->march[0]) info[5] += m.n;
+  const long in = B->tile == FUSED ? ((long)B->march[0].size() + MARCH_CELLS - 1) / MARCH_CELLS : 0;
+  info[6] = B->tile >= FLAT ? in + (B->nitems_in > 0) + (B->nitems > B->nitems_in) : 1;  // per E, H or fused pass
   info[7] = B->master->nslot;
   return IRIS_OK;
 }

@@ -1978,13 +1978,14 @@ __global__ void __launch_bounds__(FZ_X* FZ_Y, 2) k_fused(FusedArgs A) {
   fused_column<CEPS, UPML, IT>(A, S, U, blockIdx.x, blockIdx.y, z0, z1);
 }
 
-// The planes outside the UPML slabs by staged tiles (iris_march.cuh).
-template <typename TL, bool CEPS> __global__ void __launch_bounds__(MR_T, 2) k_march(MarchArgs A) {
+// Planes za..zb, outside the UPML slabs, by staged tiles (iris_march.cuh):
+// blockIdx.z covers zc planes.
+template <typename TL, bool CEPS> __global__ void __launch_bounds__(MR_T, 2) k_march(MarchArgs A, int za, int zb, int zc) {
   extern __shared__ __align__(128) unsigned char mr_dyn[];
-  const int z0 = A.za + A.zc * (int)blockIdx.z, z1 = min(z0 + A.zc - 1, A.zb);
+  const int z0 = za + zc * (int)blockIdx.z, z1 = min(z0 + zc - 1, zb);
   march_tile<TL, CEPS>(A, mr_dyn, blockIdx.x, blockIdx.y, z0, z1);
 }
-using MarchFn = void (*)(MarchArgs);
+using MarchFn = void (*)(MarchArgs, int, int, int);
 MarchFn march_kernel(int id, bool cplx) {
 #define IRIS_MARCH_K(ID, W, R) \
   if (id == ID) return cplx ? (MarchFn)k_march<MarchTile<W, R>, true> : (MarchFn)k_march<MarchTile<W, R>, false>;
@@ -2237,21 +2238,9 @@ void fused_chunks(std::vector<int>& r, int za, int zb, long tiles) {
 
 // The march of planes (za, zb, zc, n) on the engine's stream.
 void launch_march(iris_engine* E, const std::vector<int>& r) {
-  MarchArgs a{};
-  a.f = field_args<float>(E);
-  a.e_new = (float2*)E->e2;
-  a.h_new = (float2*)E->h2;
-  a.tx = E->mshape.tx;
-  a.ty = E->mshape.ty;
-  a.za = r[0], a.zb = r[1], a.zc = r[2];
-  march_kernel(E->mshape.id, E->eps_complex)<<<dim3(a.tx, a.ty, r[3]), MR_T, E->mshape.smem, E->st>>>(a);
-}
-
-// z chunks of the march: MR_CHUNK to 2 MR_CHUNK - 1 planes each.  Appends
-// (za, zb, planes per chunk, chunks) to r.
-void march_chunks(std::vector<int>& r, int za, int zb) {
-  const int len = zb - za + 1, n = std::max(1, len / MR_CHUNK), zc = (len + n - 1) / n;
-  r.insert(r.end(), {za, zb, zc, (len + zc - 1) / zc});
+  const MarchArgs a = march_args(E);
+  march_kernel(E->mshape.id, E->eps_complex)<<<dim3(a.tx, a.ty, r[3]), MR_T, E->mshape.smem, E->st>>>(a, r[0], r[1],
+                                                                                                     r[2]);
 }
 
 // One fused step into the second buffers, swap, then TF/SF and the DFT
@@ -3130,14 +3119,16 @@ int create_engine(const iris_params* pin, const double* fw, bool member, bool z_
   if (cudaSetDevice(E->device) != cudaSuccess) return bail(fail(IRIS_ECUDA, "cudaSetDevice failed"));
   if (cudaStreamCreateWithFlags(&E->st, cudaStreamNonBlocking) != cudaSuccess)
     return bail(fail(IRIS_ECUDA, "cudaStreamCreate failed"));
-  // geometry: x = 1 on a 128-byte boundary, or packed rows
+  // geometry: x = 1 on a 128-byte boundary, or packed rows (x = 1 and rows
+  // on 16-byte boundaries, for the march's copies)
   Geo& g = E->g;
   g.nx = p.nx;
   g.ny = p.ny;
   g.nz = p.nz;
   const int align = (int)(128 / E->esz);
-  g.xo = packed ? 0 : align - 1;
-  g.pitch = packed ? (long)p.nx + 2 : ((long)(g.xo + p.nx + 2) + align - 1) / align * align;
+  const int row = packed ? (E->prec == IRIS_FP32 ? 2 : 1) : align;
+  g.xo = row - 1;
+  g.pitch = ((long)(g.xo + p.nx + 2) + row - 1) / row * row;
   g.plane = g.pitch * (p.ny + 2);
   g.comp = (g.plane * (p.nz + 2) + align - 1) / align * align;
   const size_t fbytes = (size_t)3 * g.comp * E->esz;
@@ -3258,7 +3249,8 @@ int create_engine(const iris_params* pin, const double* fw, bool member, bool z_
       // the staged march where its tiles fill and 32-bit offsets reach
       if (3 * g.comp < (1L << 31)) {
         E->mshape = march_shape(p.nx, p.ny);
-        march_chunks(E->fzr[0], ia, ib);
+        const int zc = march_chunk(ib - ia + 1);
+        E->fzr[0] = {ia, ib, zc, (ib - ia + zc) / zc};
         for (bool c : {false, true})
           if (cudaFuncSetAttribute((const void*)march_kernel(E->mshape.id, c), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)E->mshape.smem) != cudaSuccess)

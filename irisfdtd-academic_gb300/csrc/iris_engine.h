@@ -214,9 +214,20 @@ template <typename T> FieldArgs<T> field_args(const iris_engine* E) {
   return a;
 }
 
+// The march's arguments for the engine's current buffers and tile shape.
+inline MarchArgs march_args(const iris_engine* E) {
+  MarchArgs a{};
+  a.f = field_args<float>(E);
+  a.e_new = (float2*)E->e2;
+  a.h_new = (float2*)E->h2;
+  a.tx = E->mshape.tx;
+  a.ty = E->mshape.ty;
+  return a;
+}
+
 // Engine lifetime.  member: a batch member (no DFT buffers of its own);
-// z_only: DFT points on the z faces only; packed: rows of nx+2 cells back to
-// back (no 128-byte alignment of x = 1), for cells whose rows are short.
+// z_only: DFT points on the z faces only; packed: rows back to back (no
+// 128-byte alignment of x = 1), for cells whose rows are short.
 int create_engine(const iris_params* pin, const double* fw, bool member, bool z_only, iris_engine** out,
                   bool packed = false);
 void free_engine(iris_engine* E);

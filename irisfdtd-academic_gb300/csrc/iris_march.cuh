@@ -39,7 +39,9 @@ namespace iris {
 // Boxes start at even elements (16 bytes): x = 1 is stored at an even index,
 // W and the pitch are even.
 
-constexpr int MR_T = 256, MR_S = 2;  // threads of a CTA (two an SM), cells a thread
+constexpr int MR_T = 512, MR_S = 1;  // threads of a CTA (two an SM), cells a thread
+// (256 threads of two cells, at 124 registers: 4.78 ms for a batch of 32 ragged
+// cells against 4.52, large planes the same)
 // Planes of a z chunk, at least: chunks this short cost 3 planes of loads each
 // but end the launch evenly and keep the CTAs at different planes (marching
 // 512x512x1024 in one chunk: 6.3 ms a pass, 31 planes a chunk 4.8, 21 4.7, 16
@@ -51,7 +53,6 @@ struct MarchArgs {
   float2* e_new;
   float2* h_new;
   int tx, ty;          // tiles of the plane
-  int za, zb, zc;      // blockIdx.z covers planes za + zc blockIdx.z on (at most zc, up to zb)
 };
 
 __device__ __forceinline__ void march_cpa16(unsigned dst, const void* src) {
@@ -339,9 +340,16 @@ __device__ __forceinline__ void march_tile(const MarchArgs& A, unsigned char* sm
     march_column<TL, CEPS, false>(A, smem, bx, by, z0, z1);
 }
 
-// The tile shapes, and the one with the fewest tiles for an nx x ny plane
-// (wider rows weigh less: their ends touch fewer sectors twice).
-#define IRIS_MARCH_SHAPES(F) F(0, 32, 14) F(1, 24, 19) F(2, 16, 29) F(3, 40, 11) F(4, 54, 8)
+// The tile shapes, and the one taken for an nx x ny plane: the fewest bytes of
+// boxes, a row counted as 24 elements longer than the tile (its halo, the
+// sectors its ends share with other tiles, and the pieces of a warp's accesses
+// a row's end splits).  512x512x256 and 256x256x512, us a pass: 54x8 1420 and
+// 662, 44x10 1410 and 662, 32x14 1428 and 675, 24x19 1482 and 697, 16x29 1547
+// and 725; wider ones (60x7, 72x6) lose on ragged planes.
+#define IRIS_MARCH_SHAPES(F) F(0, 32, 14) F(1, 24, 19) F(2, 16, 29) F(3, 44, 10) F(4, 54, 8)
+#define IRIS_MARCH_SMEM(ID, W, R) MarchTile<W, R>::SMEM,
+constexpr int MARCH_MAX_SMEM = std::max({IRIS_MARCH_SHAPES(IRIS_MARCH_SMEM) 0});
+#undef IRIS_MARCH_SMEM
 struct MarchShape {
   int id = -1, tx = 0, ty = 0;  // id < 0: none
   size_t smem = 0;
@@ -352,7 +360,7 @@ inline MarchShape march_shape(int nx, int ny) {
 #define IRIS_MARCH_TRY(ID, W, R)                                        \
   {                                                                     \
     const int tx = (nx + W - 1) / W, ty = (ny + R - 1) / R;             \
-    const double c = (double)tx * ty * (1.0 + 1.0 / W);                 \
+    const double c = (double)tx * ty * (W + 24) * (R + 1.5);            \
     if (c < cost) {                                                     \
       cost = c;                                                         \
       best.id = ID, best.tx = tx, best.ty = ty;                         \
@@ -363,10 +371,10 @@ inline MarchShape march_shape(int nx, int ny) {
 #undef IRIS_MARCH_TRY
   return best;
 }
-// Share of the march's threads that own a cell of the plane.
-inline double march_fill(int nx, int ny) {
-  const MarchShape s = march_shape(nx, ny);
-  return (double)nx * ny / ((double)s.tx * s.ty * MR_T * MR_S);
+// Planes of a z chunk of len planes: MR_CHUNK to 2 MR_CHUNK - 1, or len.
+inline int march_chunk(int len) {
+  const int n = std::max(1, len / MR_CHUNK);
+  return (len + n - 1) / n;
 }
 
 }  // namespace iris

@@ -49,3 +49,35 @@ def test_march_equals_split(iris, tmp_path, nx, ny, planes, lossy):
         e.close()
     for k, (a, b) in enumerate(zip(*out)):
         assert np.array_equal(a, b), (k, int(np.sum(a != b)))
+
+
+def test_march_batch_equals_engines(iris, tmp_path):
+    """Cells of every tile shape, more than one launch takes, one without
+    planes to march and one with a complex material among real ones."""
+    sizes = [(c[0], c[1], 6 + c[2]) for c in CASES] * 3
+    sizes[7] = (9, 5, 10)
+    ps, mats = [], []
+    r = np.random.default_rng(8)
+    for c, (nx, ny, nz) in enumerate(sizes):
+        w = cfg.Workload("march", nx, ny, nz, 3, 5 if c == 7 else nz - 2, 5, 1, 2.25, 0, 4,
+                         (1, nx, 1, ny, 4, 4), 5, 9)
+        p, fw, _ = iris.setparam(cfg.write_input(str(tmp_path / "in.dat"), w, i_pol=2))
+        p.akx_re, p.aky_re, p.precision = 0.3, -0.7, iris.FP32
+        ps.append(p)
+        shape = (p.hf - p.hi + 3, ny + 2, nx + 2)
+        mats.append(1.0 / r.uniform(1.0, 6.0, shape) + (1j * r.uniform(-0.02, 0.02, shape) if c == 5 else 0.0))
+    out = []
+    b = iris.Batch(ps, fw, precision=iris.FP32, dft_faces=iris.DFT_Z)
+    for c, m in enumerate(mats):
+        b.set_material(c, m)
+    b.set_tile(7)  # the fused work list
+    b.step(150, 7)
+    for c, p in enumerate(ps):
+        e = iris.Engine(p, fw, precision=iris.FP32, stencil=iris.STENCIL_SPLIT)
+        e.set_material(mats[c])
+        e.step(150, 7)
+        for which in (iris.E, iris.H):
+            assert np.array_equal(interior(b.get_field(c, which), p), interior(e.get_field(which), p)), (c, which)
+        assert np.any(interior(b.get_field(c, iris.E), p))
+        e.close()
+    b.close()
