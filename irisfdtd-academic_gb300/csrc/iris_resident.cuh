@@ -551,7 +551,7 @@ __device__ __forceinline__ double res_dl2(const double2* f, int i, int p) { retu
 __device__ __forceinline__ double res_ds(const double2* f, int i, int p) { return ((const double*)(f + i))[p]; }
 // Part p of ph * w, as cmul rounds it.
 __device__ __forceinline__ double res_dph(cx<double> ph, cx<double> w, int p) {
-  return p == 0 ? ds(dm(ph.re, w.re), dm(ph.im, w.im)) : da(dm(ph.re, w.im), dm(ph.im, w.re));
+  return p == 0 ? axmby_(ph.re, w.re, ph.im, w.im) : axpby_(ph.re, w.im, ph.im, w.re);
 }
 // The other part of the same cell and component: on the neighbouring lane
 // (items come in pairs and both lanes of a pair take the same branches).
@@ -596,20 +596,20 @@ __device__ __forceinline__ void res_e64(const ResArgs<double>& A, const ResView<
     const double* cf = u.cf + k;
     double* D = (double*)(u.f + k * u.pc + x) + p;
     const double dold = *D;
-    const double dn = da(dm(cf[CD_A], dold), dm(cf[CD_B], dm(a.eps0sq, c)));
+    const double dn = axpby_(cf[CD_A], dold, cf[CD_B], dm(a.eps0sq, c));
     *D = dn;
-    e = da(dm(cf[CE_A], e), dm(cf[CE_B], ds(dm(cf[C_FP], dn), dm(cf[C_FM], dold))));
+    e = axpby_(cf[CE_A], e, cf[CE_B], axmby_(cf[C_FP], dn, cf[C_FM], dold));
   } else if (r.fl & RF_MAT) {
     const int ie = gi - a.hi * (int)g.plane;
     if (CEPS) {
       const double2 w = a.eps_c[ie];
       const double o = curl(p ^ 1);
-      e = da(e, res_dph(cx<double>{w.x, w.y}, p == 0 ? cx<double>{c, o} : cx<double>{o, c}, p));
+      e = axpy_(w.x, c, axpy_(p == 0 ? -w.y : w.y, o, e));
     } else {
-      e = da(e, dm(a.eps_r[ie], c));
+      e = axpy_(a.eps_r[ie], c, e);
     }
   } else {
-    e = da(e, dm(r.fl & RF_SUB ? a.m3 : a.m1, c));
+    e = axpy_(r.fl & RF_SUB ? a.m3 : a.m1, c, e);
   }
   if (!(NC == 5 && k == 0)) ((double*)(v.e(k) + li))[p] = e;
   if ((r.fl & RF_PUB) || (NC == 5 && k == 0)) ((double*)(a.e + k * cp + gi))[p] = e;
@@ -650,11 +650,11 @@ __device__ __forceinline__ void res_h64(const ResArgs<double>& A, const ResView<
     const double* cf = u.cf + k;
     double* B = (double*)(u.f + k * u.pc + x) + p;
     const double bold = *B;
-    const double bn = ds(dm(cf[CD_A], bold), dm(cf[CB_B], c));
+    const double bn = axmby_(cf[CD_A], bold, cf[CB_B], c);
     *B = bn;
-    h = da(dm(cf[CE_A], h), dm(cf[CH_B], ds(dm(cf[C_FP], bn), dm(cf[C_FM], bold))));
+    h = axpby_(cf[CE_A], h, cf[CH_B], axmby_(cf[C_FP], bn, cf[C_FM], bold));
   } else {
-    h = ds(h, dm(a.dtcq2, c));
+    h = ymax_(h, a.dtcq2, c);
   }
   const bool ck = (r.fl & RF_CORR) && k == A.s.cH;
   auto fix = [&](double q, int ix) {
