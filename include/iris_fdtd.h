@@ -325,6 +325,9 @@ int iris_set_pml_c(iris_engine* eng, int which, int slab, const double* c);
  */
 int iris_get_plane(iris_engine* eng, int which, int axis, int index, int lo1, int hi1, int lo2, int hi2,
                    double* re, double* im);
+/* The same as interleaved (re, im) doubles, through the staging buffer of
+ * iris_get_field_c straight into c. */
+int iris_get_plane_c(iris_engine* eng, int which, int axis, int index, int lo1, int hi1, int lo2, int hi2, double* c);
 
 /*
  * DFT accumulator emg(j)%fdata(i_pts, iw) of box (0/1) and face pair

@@ -266,10 +266,10 @@ class Engine:
         """One plane (axis 1, 2, 3 = x, y, z = index) over the in-plane ranges
         r1 = (lo, hi), r2 = (lo, hi), as complex [i2, i1, component]."""
         n1, n2 = r1[1] - r1[0] + 1, r2[1] - r2[0] + 1
-        re, im = np.empty(3 * n1 * n2), np.empty(3 * n1 * n2)
-        check(self.L.iris_get_plane(self.h, which, axis, index, r1[0], r1[1], r2[0], r2[1], _dp(re), _dp(im)),
-              "iris_get_plane")
-        return (re + 1j * im).reshape(n2, n1, 3)
+        a = np.empty(max(0, 3 * n1 * n2), dtype=np.complex128)
+        check(self.L.iris_get_plane_c(self.h, which, axis, index, r1[0], r1[1], r2[0], r2[1],
+                                      a.ctypes.data_as(ctypes.POINTER(ctypes.c_double))), "iris_get_plane_c")
+        return a.reshape(n2, n1, 3)
 
     # -- instrumentation
     KERNELS = ("update_e", "update_h", "tfsf", "dft_gather", "dft_block", "flux", "fused_eh", "persistent")

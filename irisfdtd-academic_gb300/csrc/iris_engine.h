@@ -6,6 +6,8 @@
 #include <cuda_runtime.h>
 
 #include <functional>
+#include <memory>
+#include <new>
 #include <string>
 #include <utility>
 #include <vector>

@@ -116,7 +116,7 @@ EXPORTS = [
     "iris_dft_commit", "iris_material_spheres", "iris_material_pattern", "iris_material_design",
     "iris_get_material", "iris_batch_material_pattern", "iris_write_scatt", "iris_get_field", "iris_set_field", "iris_get_pml", "iris_set_pml",
     "iris_get_field_c", "iris_set_field_c", "iris_get_pml_c", "iris_set_pml_c",
-    "iris_get_fdata", "iris_get_plane", "iris_apply", "iris_run_input", "iris_timing", "iris_timing_read", "iris_info",
+    "iris_get_fdata", "iris_get_plane", "iris_get_plane_c", "iris_apply", "iris_run_input", "iris_timing", "iris_timing_read", "iris_info",
     "iris_bounds_check",
     "iris_dft_block_noalloc", "iris_batch_create", "iris_batch_destroy", "iris_batch_set_material",
     "iris_batch_step", "iris_batch_flux", "iris_batch_dft_commit", "iris_batch_get_field", "iris_batch_tune",
@@ -173,6 +173,7 @@ def lib():
     L.iris_set_pml_c.argtypes = [vp, ip, ip, dp]
     L.iris_get_fdata.argtypes = [vp, ip, ip, dp, dp, ctypes.POINTER(ctypes.c_long)]
     L.iris_get_plane.argtypes = [vp, ip, ip, ip, ip, ip, ip, ip, dp, dp]
+    L.iris_get_plane_c.argtypes = [vp, ip, ip, ip, ip, ip, ip, ip, dp]
     L.iris_apply.argtypes = [vp, ip, ip]
     L.iris_run_input.argtypes = [cp, ip]
     L.iris_timing.argtypes = [vp, ip]
