@@ -336,20 +336,20 @@ __device__ __forceinline__ void h_cell(const FieldArgs<T>& a, int x, int y, int 
 // Split E pass of one cell: e_cell in place + bc_{x,y,z}max_bloch
 // (code/boundary.f90:193-216,257-284,321-348) for the E ghosts.  MASK: the
 // components computed and stored (bit k: E_{k+1}); the components of a cell
-// are independent, so a cell may be split over threads.
-template <typename T, bool CEPS, bool UPML = true, int MASK = 7>
-__device__ __forceinline__ void e_split_cell(const FieldArgs<T>& a, int x, int y, int z) {
+// are independent, so a cell may be split over threads.  XG = false: the
+// caller stores the x image from the new E it is given back.
+template <typename T, bool CEPS, bool UPML = true, int MASK = 7, bool XG = true>
+__device__ __forceinline__ void e_split_cell(const FieldArgs<T>& a, int x, int y, int z, cx<T> (&e)[3]) {
   using V = typename V2<T>::t;
   const Geo& g = a.g;
   const long i = g.at(x, y, z);
   if (!bc_ok(x >= 1 && x <= g.nx && y >= 1 && y <= g.ny && z >= 1 && z <= g.nz, BC_E_CELL, i)) return;
   V* E[3] = {a.e, a.e + g.comp, a.e + 2 * g.comp};
-  cx<T> e[3];
   e_cell<T, CEPS, MASK, UPML>(a, a.pml_d, x, y, z, e);
 #pragma unroll
   for (int k = 0; k < 3; ++k)
     if (MASK & (1 << k)) st<T>(E[k] + i, e[k]);
-  if (x == 1) {
+  if (XG && x == 1) {
     const long j = g.at(g.nx + 1, y, z);
 #pragma unroll
     for (int k = 0; k < 3; ++k)
@@ -369,19 +369,26 @@ __device__ __forceinline__ void e_split_cell(const FieldArgs<T>& a, int x, int y
   }
 }
 
+template <typename T, bool CEPS, bool UPML = true, int MASK = 7>
+__device__ __forceinline__ void e_split_cell(const FieldArgs<T>& a, int x, int y, int z) {
+  cx<T> e[3];
+  e_split_cell<T, CEPS, UPML, MASK, true>(a, x, y, z, e);
+}
+
 // Split H pass of one cell: h_cell in place + bc_{x,y,z}min_bloch
 // (code/boundary.f90:163-187,224-251,288-315) for the H ghosts and the E
 // ghosts at 0.  The ghosts at nx+1/ny+1/nz+1 of H are never read by any
-// operator and are not maintained.
-template <typename T, bool UPML = true, int MASK = 7>
-__device__ __forceinline__ void h_split_cell(const FieldArgs<T>& a, int x, int y, int z) {
+// operator and are not maintained.  XG = false: the caller stores the x images
+// from the E (v[0..2]) and new H (v[3..5]) it is given back.
+template <typename T, bool UPML = true, int MASK = 7, bool XG = true>
+__device__ __forceinline__ void h_split_cell(const FieldArgs<T>& a, int x, int y, int z, cx<T> (&v)[6]) {
   using V = typename V2<T>::t;
   const Geo& g = a.g;
   const long i = g.at(x, y, z);
   if (!bc_ok(x >= 1 && x <= g.nx && y >= 1 && y <= g.ny && z >= 1 && z <= g.nz, BC_H_CELL, i)) return;
   V* Ec[3] = {a.e, a.e + g.comp, a.e + 2 * g.comp};
   V* H[3] = {a.h, a.h + g.comp, a.h + 2 * g.comp};
-  cx<T> ev[3], xp[3], yp[3], zp[3], h[3];
+  cx<T>*ev = v, *h = v + 3, xp[3], yp[3], zp[3];
 #pragma unroll
   for (int k = 0; k < 3; ++k) ev[k] = ld<T>(Ec[k] + i);
   xp[1] = ld<T>(Ec[1] + i + 1);
@@ -394,7 +401,7 @@ __device__ __forceinline__ void h_split_cell(const FieldArgs<T>& a, int x, int y
 #pragma unroll
   for (int k = 0; k < 3; ++k)
     if (MASK & (1 << k)) st<T>(H[k] + i, h[k]);
-  if (x == g.nx) {
+  if (XG && x == g.nx) {
     const long j = g.at(0, y, z);
 #pragma unroll
     for (int k = 0; k < 3; ++k)
@@ -420,6 +427,50 @@ __device__ __forceinline__ void h_split_cell(const FieldArgs<T>& a, int x, int y
         st<T>(Ec[k] + j, cphase(a.pzm, ev[k]));
         st<T>(H[k] + j, cphase(a.pzm, h[k]));
       }
+  }
+}
+
+template <typename T, bool UPML = true, int MASK = 7>
+__device__ __forceinline__ void h_split_cell(const FieldArgs<T>& a, int x, int y, int z) {
+  cx<T> v[6];
+  h_split_cell<T, UPML, MASK, true>(a, x, y, z, v);
+}
+
+// x images of a warp's border cells in FP64, by the whole warp (all its lanes
+// call): lane l forms number l (component l / 2, part l % 2) of the NV values
+// of a lane with own set, two FP64 instructions instead of the 4 NV that the
+// lane would take the warp through alone; with 2 NV such lanes or more those
+// are as few.  j: storage index of the lane's image; v[0..2] go to the three
+// components of f, v[3..5] to those of f2.
+template <int NV>
+__device__ __forceinline__ void warp_images(bool own, cx<double> ph, const cx<double> (&v)[NV], long j, double2* f,
+                                            double2* f2, long comp) {
+  unsigned m = __ballot_sync(0xffffffffu, own);
+  if (m == 0) return;
+  if ((ph.re == 1.0 && ph.im == 0.0) || __popc(m) >= 2 * NV) {
+    if (own)
+#pragma unroll
+      for (int k = 0; k < NV; ++k) st<double>((k < 3 ? f : f2) + (k % 3) * comp + j, cphase(ph, v[k]));
+    return;
+  }
+  const int l = threadIdx.x & 31, p = l & 1, kk = l >> 1;
+  const double pi = p ? ph.im : -ph.im;
+  for (; m; m &= m - 1) {
+    const int s = __ffs(m) - 1;
+    const long js = __shfl_sync(0xffffffffu, j, s);
+    double x = 0.0, y = 0.0;
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+      const double re = __shfl_sync(0xffffffffu, v[k].re, s), im = __shfl_sync(0xffffffffu, v[k].im, s);
+      if (k == kk) {
+        x = p ? im : re;
+        y = p ? re : im;
+      }
+    }
+    if (kk < NV) {
+      double2* d = (kk < 3 ? f + kk * comp : f2 + (kk - 3) * comp) + js;
+      ((double*)d)[p] = axpby_(ph.re, x, pi, y);
+    }
   }
 }
 

@@ -42,22 +42,46 @@
 namespace iris {
 namespace {
 
-template <typename T, bool CEPS>
-__global__ void __launch_bounds__(256) k_update_e(FieldArgs<T> a) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x + 1;
-  const int y = blockIdx.y * blockDim.y + threadIdx.y + 1;
-  const int z = blockIdx.z * blockDim.z + threadIdx.z + 1;
-  if (x > a.g.nx || y > a.g.ny || z > a.g.nz) return;
-  e_split_cell<T, CEPS>(a, x, y, z);
+// The FP64 split passes: a thread a cell, in (z, y, x) order.  They are bound
+// by FP64 issue (85 % of the pipe at 128x128x160), and a warp's FP64
+// instruction takes the same 64 cycles with any number of lanes active: so rows
+// are packed into full warps and the x images formed by the whole warp.
+// 128x128x160 at a Bloch phase: 402 us a step before, 362 so; 90x90x120 188
+// and 159.
+template <bool CEPS> __global__ void __launch_bounds__(256) k_update_e64(FieldArgs<double> a) {
+  const unsigned L = blockIdx.x * 256u + threadIdx.x, nx = (unsigned)a.g.nx, nxy = nx * (unsigned)a.g.ny;
+  const unsigned zq = L / nxy, r = L - zq * nxy, yq = r / nx;
+  const int x = (int)(r - yq * nx) + 1, y = (int)yq + 1, z = (int)zq + 1;
+  const bool in = z <= a.g.nz;
+  cx<double> e[3] = {};
+  if (in) e_split_cell<double, CEPS, true, 7, false>(a, x, y, z, e);
+  warp_images<3>(in && x == 1, a.pxp, e, a.g.at(a.g.nx + 1, y, z), a.e, a.e, a.g.comp);
+}
+__global__ void __launch_bounds__(256) k_update_h64(FieldArgs<double> a) {
+  const unsigned L = blockIdx.x * 256u + threadIdx.x, nx = (unsigned)a.g.nx, nxy = nx * (unsigned)a.g.ny;
+  const unsigned zq = L / nxy, r = L - zq * nxy, yq = r / nx;
+  const int x = (int)(r - yq * nx) + 1, y = (int)yq + 1, z = (int)zq + 1;
+  const bool in = z <= a.g.nz;
+  cx<double> v[6] = {};
+  if (in) h_split_cell<double, true, 7, false>(a, x, y, z, v);
+  warp_images<6>(in && x == a.g.nx, a.pxm, v, a.g.at(0, y, z), a.e, a.h, a.g.comp);
 }
 
-template <typename T>
-__global__ void __launch_bounds__(256) k_update_h(FieldArgs<T> a) {
+// The FP32 split passes.
+template <bool CEPS> __global__ void __launch_bounds__(256) k_update_e(FieldArgs<float> a) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x + 1;
   const int y = blockIdx.y * blockDim.y + threadIdx.y + 1;
   const int z = blockIdx.z * blockDim.z + threadIdx.z + 1;
   if (x > a.g.nx || y > a.g.ny || z > a.g.nz) return;
-  h_split_cell<T>(a, x, y, z);
+  e_split_cell<float, CEPS>(a, x, y, z);
+}
+
+__global__ void __launch_bounds__(256) k_update_h(FieldArgs<float> a) {
+  const int x = blockIdx.x * blockDim.x + threadIdx.x + 1;
+  const int y = blockIdx.y * blockDim.y + threadIdx.y + 1;
+  const int z = blockIdx.z * blockDim.z + threadIdx.z + 1;
+  if (x > a.g.nx || y > a.g.ny || z > a.g.nz) return;
+  h_split_cell<float>(a, x, y, z);
 }
 
 // The device-resident step base of captured graphs.
@@ -2137,6 +2161,9 @@ int validate(const iris_params& p) {
   return IRIS_OK;
 }
 
+// CTAs of the FP64 split passes (memory keeps the cells below 2^32 - 256).
+unsigned blocks64(const iris_engine* E) { return (unsigned)(((long)E->p.nx * E->p.ny * E->p.nz + 255) / 256); }
+
 template <typename T> void launch_e(iris_engine* E) {
   KTimer tm(E, IRIS_KC_E);
   FieldArgs<T> a = field_args<T>(E);
@@ -2145,9 +2172,12 @@ template <typename T> void launch_e(iris_engine* E) {
       k_stream_e<<<E->sgrd, dim3(SX, SY), STREAM_SMEM_E, E->st>>>(a, E->d_err);
       return;
     }
+    if (E->eps_complex) k_update_e<true><<<E->grd, E->blk, 0, E->st>>>(a);
+    else k_update_e<false><<<E->grd, E->blk, 0, E->st>>>(a);
+  } else {
+    if (E->eps_complex) k_update_e64<true><<<blocks64(E), 256, 0, E->st>>>(a);
+    else k_update_e64<false><<<blocks64(E), 256, 0, E->st>>>(a);
   }
-  if (E->eps_complex) k_update_e<T, true><<<E->grd, E->blk, 0, E->st>>>(a);
-  else k_update_e<T, false><<<E->grd, E->blk, 0, E->st>>>(a);
 }
 template <typename T> void launch_h(iris_engine* E) {
   KTimer tm(E, IRIS_KC_H);
@@ -2157,7 +2187,8 @@ template <typename T> void launch_h(iris_engine* E) {
       return;
     }
   }
-  k_update_h<T><<<E->grd, E->blk, 0, E->st>>>(field_args<T>(E));
+  if constexpr (std::is_same<T, float>::value) k_update_h<<<E->grd, E->blk, 0, E->st>>>(field_args<float>(E));
+  else k_update_h64<<<blocks64(E), 256, 0, E->st>>>(field_args<double>(E));
 }
 // The TF/SF table of steps it .. it+n-1 (at most tfv_cap), from *itp on when
 // itp is given.
@@ -2488,6 +2519,27 @@ int res_setup(iris_engine* E) {
   CK(cudaMalloc(&E->d_rflag, sizeof(unsigned) * RES_FLAG_STRIDE * G));
   E->res = true;
   return IRIS_OK;
+}
+
+// Microseconds of an FP64 step, as measured on GB300: the resident kernel by
+// its busiest CTA, 18 ns a cell and twice that in the UPML (256x4x340, 2290
+// cells a CTA, 47 us; 2600x1x16, a UPML row of 2600 on a CTA, 95); k_tiny 0.24
+// ns a cell and its barriers (20x20x1000 93, 128x128x60 194); the split passes
+// 0.15 to 0.2 ns a cell and the launches (2600x1x16 36, 20x20x1000 71,
+// 70x70x70 70, 128x128x60 160).
+double res_us64(const iris_engine* E) {
+  const iris_params& p = E->p;
+  long most = 0;
+  for (const ResCta& c : E->res_cta) {
+    long n = 0;
+    for (long r = c.r0; r < c.r1; ++r) n += r / p.ny < p.pmlzi || r / p.ny + 1 >= p.pmlzf ? 2 : 1;
+    most = std::max(most, n * p.nx);
+  }
+  return 5.0 + 0.018 * most;
+}
+double tiny_us64(const iris_engine* E) { return 5.0 + 2.4e-4 * E->p.nx * E->p.ny * E->p.nz; }
+double split_us64(const iris_engine* E) {
+  return std::max(36.0, 10.0 + 1.8e-4 * E->p.nx * E->p.ny * E->p.nz);
 }
 
 // The sample points of every CTA, E then H, each in ring order: shared-memory
@@ -3178,9 +3230,8 @@ int create_engine(const iris_params* pin, const double* fw, bool member, bool z_
   E->src = make_src(p);
   // Small grids step with the persistent kernel (asked for, or by default
   // when the device runs cooperative launches: FP64 grids of at most
-  // IRIS_PERSISTENT_MAX_CELLS cells, FP32 grids of at most
-  // IRIS_PERSISTENT_MAX_CELLS_FP32: up to those sizes it steps faster than
-  // the split passes); otherwise FP32 steps with the fused E+H pass unless the split or
+  // IRIS_PERSISTENT_MAX_CELLS cells that it is estimated to step faster,
+  // FP32 grids of at most IRIS_PERSISTENT_MAX_CELLS_FP32); otherwise FP32 steps with the fused E+H pass unless the split or
   // streamed passes are asked for, or unless the fused pass's 32 x 16 tiles
   // would leave more than half of their threads idle on the grid's x-y
   // plane (rows or columns short of a tile: the split passes then); FP64
@@ -3226,6 +3277,11 @@ int create_engine(const iris_params* pin, const double* fw, bool member, bool z_
   if (E->persist) {
     rc = res_setup(E);
     if (rc) return bail(rc);
+    if (E->prec == IRIS_FP64) {
+      const double res = E->res ? res_us64(E) : 1e300, tiny = tiny_us64(E);
+      if (res > tiny) E->res = false;
+      if (p.stencil == IRIS_STENCIL_DEFAULT && std::min(res, tiny) > split_us64(E)) E->persist = E->res = false;
+    }
   }
   E->fused = !E->persist && E->prec == IRIS_FP32 &&
              (p.stencil == IRIS_STENCIL_FUSED || (p.stencil == IRIS_STENCIL_DEFAULT && fused_fill(p.nx, p.ny) >= 0.5));
