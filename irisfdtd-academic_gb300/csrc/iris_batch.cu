@@ -184,8 +184,8 @@ __global__ void __launch_bounds__(FZ_X* FZ_Y, 2) k_batch_fused(const FusedArgs* 
 // there, or held in registers, in every plane: 4.44 ms against 4.20 for 32
 // ragged cells of 182 million points, whose E and H passes over flat runs take
 // 5.26; their 96 bytes a point take 2.6 at the measured copy bandwidth.  The
-// UPML slabs (k_batch_fused) and the tiles' unfilled threads (a fifth) make
-// up most of the difference.
+// UPML slabs and the tiles' unfilled threads (a fifth) make up most of the
+// difference.
 constexpr int MARCH_CELLS = 48;
 struct MarchCell {
   MarchArgs a;
@@ -208,6 +208,34 @@ template <bool CEPS> __global__ void __launch_bounds__(MR_T, 2) k_batch_march(co
     break;
   switch (c.shape) { IRIS_MARCH_SHAPES(IRIS_MARCH_CASE) }
 #undef IRIS_MARCH_CASE
+}
+
+// The slabs, likewise: CTAs (x tile, y tile, z chunk), the first nc0 chunks of
+// planes za0..zb0, the rest of za1..zb1.
+struct SlabCell {
+  MarchSlabArgs a;
+  int za0, zb0, zc0, nc0, za1, zb1, zc1, n;
+  int shape;
+};
+struct SlabCells {
+  SlabCell c[MARCH_CELLS];
+};
+template <bool CEPS> __global__ void __launch_bounds__(MS_T, 2) k_batch_slab(const __grid_constant__ SlabCells P) {
+  extern __shared__ __align__(128) unsigned char mr_dyn[];
+  const SlabCell& c = P.c[blockIdx.y];
+  if ((int)blockIdx.x >= c.n) return;
+  const int tiles = c.a.m.tx * c.a.m.ty, iz = blockIdx.x / tiles, t = blockIdx.x - iz * tiles;
+  const int by = t / c.a.m.tx, bx = t - by * c.a.m.tx;
+  const bool r0 = iz < c.nc0;
+  const int z0 = r0 ? c.za0 + iz * c.zc0 : c.za1 + (iz - c.nc0) * c.zc1;
+  const int z1 = min(z0 + (r0 ? c.zc0 : c.zc1) - 1, r0 ? c.zb0 : c.zb1);
+#define IRIS_SLAB_CASE(ID, W, R)                                                                             \
+  case ID:                                                                                                   \
+    if (CEPS && c.a.m.f.eps_c) march_tile<SlabTile<W, R>, true>(c.a.m, mr_dyn, bx, by, z0, z1, c.a.d_new);    \
+    else march_tile<SlabTile<W, R>, false>(c.a.m, mr_dyn, bx, by, z0, z1, c.a.d_new);                        \
+    break;
+  switch (c.shape) { IRIS_SLAB_SHAPES(IRIS_SLAB_CASE) }
+#undef IRIS_SLAB_CASE
 }
 
 // The TF/SF corrections of steps it0 .. it0+n-1 (from *itp on when given) for
@@ -272,11 +300,12 @@ struct iris_batch {
   bool second = false;
   int parity = 0;
   void* d_fargs = nullptr;
-  // the planes outside the slabs of the cells that march (all but those too
-  // large for its 32-bit offsets, which have FUSED items), per parity; the
-  // slab launch runs on st2, as in the single engine
+  // the planes outside the slabs and the slabs of the cells that march (all
+  // but those too large for its 32-bit offsets, which have FUSED items), per
+  // parity; the slabs run on st2, as in the single engine
   std::vector<MarchCell> march[2];
-  size_t march_smem = 0;
+  std::vector<SlabCell> slab[2];
+  size_t march_smem = 0, slab_smem = 0;
   cudaStream_t st2 = nullptr;
   cudaEvent_t fork = nullptr, join = nullptr;
   FItem* d_fitems = nullptr;
@@ -310,16 +339,32 @@ void swap_sets(iris_engine* E) {
 
 // The march's cells (second buffers present), for both buffer parities.
 void batch_march_cells(iris_batch* B) {
-  B->march_smem = 0;
+  B->march_smem = B->slab_smem = 0;
   for (int q = 0; q < 2; ++q) {
     B->march[q].clear();
+    B->slab[q].clear();
     for (iris_engine* E : B->cells) {
-      const int ia = E->p.pmlzi + 1, ib = E->p.pmlzf - 2;
-      if (ib < ia || E->mshape.id < 0) continue;
+      if (E->mshape.id < 0) continue;
+      const int ia = E->p.pmlzi + 1, ib = E->p.pmlzf - 2, nz = E->p.nz;
       if (q != B->parity) swap_sets(E);
       MarchCell m{};
       m.a = march_args(E);
+      SlabCell s{};
+      s.a = march_slab_args(E);
       if (q != B->parity) swap_sets(E);
+      // planes 1 .. ia-1 and ib+1 .. nz, or all
+      s.za0 = 1, s.zb0 = ib >= ia ? ia - 1 : nz;
+      s.za1 = ib + 1, s.zb1 = ib >= ia ? nz : ib;
+      const int l0 = s.zb0 - s.za0 + 1, l1 = s.zb1 - s.za1 + 1;
+      s.zc0 = slab_chunk(l0), s.zc1 = slab_chunk(l1);
+      s.nc0 = l0 > 0 ? (l0 + s.zc0 - 1) / s.zc0 : 0;
+      s.n = s.a.m.tx * s.a.m.ty * (s.nc0 + (l1 > 0 ? (l1 + s.zc1 - 1) / s.zc1 : 0));
+      s.shape = E->sshape.id;
+      if (s.n > 0) {
+        B->slab[q].push_back(s);
+        B->slab_smem = std::max(B->slab_smem, E->sshape.smem);
+      }
+      if (ib < ia) continue;
       m.za = ia, m.zb = ib, m.zc = march_chunk(ib - ia + 1);
       m.n = m.a.tx * m.a.ty * ((ib - ia + m.zc) / m.zc);
       m.shape = E->mshape.id;
@@ -402,7 +447,10 @@ int batch_second_buffers(iris_batch* B) {
     CK(cudaEventCreateWithFlags(&B->join, cudaEventDisableTiming));
   }
   for (iris_engine* E : B->cells) {
-    if (3 * E->g.comp < (1L << 31)) E->mshape = march_shape(E->p.nx, E->p.ny);
+    if (3 * E->g.comp < (1L << 31)) {
+      E->mshape = march_shape(E->p.nx, E->p.ny);
+      E->sshape = slab_shape(E->p.nx, E->p.ny);
+    }
     const size_t fbytes = (size_t)3 * E->g.comp * E->esz;
     if (!E->e2) CK(cudaMalloc(&E->e2, fbytes));
     if (!E->h2) CK(cudaMalloc(&E->h2, fbytes));
@@ -418,13 +466,14 @@ int batch_second_buffers(iris_batch* B) {
   return batch_upload_args(B);
 }
 
-// FUSED items: the planes outside the UPML slabs (stopping at pmlzf-2, as the
-// single-engine launch does) of the cells that do not march, in chunks of
-// FB_CHUNK, then every cell's two slabs each with the plane next to it;
-// within a chunk, tile rows of the cell in order.
+// FUSED items, of the cells that do not march: the planes outside the UPML
+// slabs (stopping at pmlzf-2, as the single-engine launch does) in chunks of
+// FB_CHUNK, then the two slabs each with the plane next to it; within a chunk,
+// tile rows of the cell in order.
 int batch_build_fused_items(iris_batch* B) {
   std::vector<FItem> in, slab;
   for (int c = 0; c < B->n; ++c) {
+    if (B->cells[c]->mshape.id >= 0) continue;
     const iris_params& p = B->cells[c]->p;
     const int tx = (p.nx + FZ_OX - 1) / FZ_OX, ty = (p.ny + FZ_OY - 1) / FZ_OY;
     auto add = [&](std::vector<FItem>& v, int za, int zb, int len) {
@@ -434,7 +483,7 @@ int batch_build_fused_items(iris_batch* B) {
     };
     const int ia = p.pmlzi + 1, ib = p.pmlzf - 2;
     if (ib >= ia) {
-      if (B->cells[c]->mshape.id < 0) add(in, ia, ib, FB_CHUNK);
+      add(in, ia, ib, FB_CHUNK);
       add(slab, 1, ia - 1, p.nz);
       add(slab, ib + 1, p.nz, p.nz);
     } else {
@@ -447,6 +496,8 @@ int batch_build_fused_items(iris_batch* B) {
     CK(cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FZ_UPML_SMEM));
   for (const void* kf : {(const void*)k_batch_march<false>, (const void*)k_batch_march<true>})
     CK(cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, MARCH_MAX_SMEM));
+  for (const void* kf : {(const void*)k_batch_slab<false>, (const void*)k_batch_slab<true>})
+    CK(cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, SLAB_MAX_SMEM));
   graph_reset(B->master);
   if (B->d_fitems) cudaFree(B->d_fitems);
   B->d_fitems = nullptr;
@@ -577,25 +628,33 @@ template <bool CEPS> void launch_batch_fused(iris_batch* B) {
   };
   static int per_in = 0, per_slab = 0;
   KTimer tm(M, IRIS_KC_FUSED);
-  const bool both = nslab > 0 && (nbig > 0 || !mc.empty());
+  const std::vector<SlabCell>& sc = B->slab[B->parity];
+  const bool both = (nslab > 0 || !sc.empty()) && (nbig > 0 || !mc.empty());
+  cudaStream_t st2 = both ? B->st2 : M->st;
   if (both) {
     cudaEventRecord(B->fork, M->st);
     cudaStreamWaitEvent(B->st2, B->fork, 0);
   }
+  // up to MARCH_CELLS cells a launch
+  auto each = [](auto& P, const auto& v, auto launch) {
+    for (size_t i = 0; i < v.size(); i += MARCH_CELLS) {
+      const size_t n = std::min<size_t>(MARCH_CELLS, v.size() - i);
+      int ctas = 0;
+      for (size_t j = 0; j < n; ++j) {
+        P.c[j] = v[i + j];
+        ctas = std::max(ctas, P.c[j].n);
+      }
+      launch(dim3(ctas, (unsigned)n), P);
+    }
+  };
+  SlabCells S;
+  MarchCells P;
+  each(S, sc, [&](dim3 g, const SlabCells& c) { k_batch_slab<CEPS><<<g, MS_T, B->slab_smem, st2>>>(c); });
   if (nslab > 0) {
     const unsigned g = ctas((const void*)k_batch_fused<CEPS, true>, FZ_UPML_SMEM, nslab, per_slab);
-    k_batch_fused<CEPS, true><<<g, blk, FZ_UPML_SMEM, both ? B->st2 : M->st>>>(args, B->d_fitems + B->nitems_in, nslab);
+    k_batch_fused<CEPS, true><<<g, blk, FZ_UPML_SMEM, st2>>>(args, B->d_fitems + B->nitems_in, nslab);
   }
-  for (size_t i = 0; i < mc.size(); i += MARCH_CELLS) {
-    MarchCells P;
-    const size_t n = std::min<size_t>(MARCH_CELLS, mc.size() - i);
-    int ctas = 0;
-    for (size_t j = 0; j < n; ++j) {
-      P.c[j] = mc[i + j];
-      ctas = std::max(ctas, P.c[j].n);
-    }
-    k_batch_march<CEPS><<<dim3(ctas, (unsigned)n), MR_T, B->march_smem, M->st>>>(P);
-  }
+  each(P, mc, [&](dim3 g, const MarchCells& c) { k_batch_march<CEPS><<<g, MR_T, B->march_smem, M->st>>>(c); });
   if (nbig > 0) {
     const unsigned g = ctas((const void*)k_batch_fused<CEPS, false>, 0, nbig, per_in);
     k_batch_fused<CEPS, false><<<g, blk, 0, M->st>>>(args, B->d_fitems, nbig);
@@ -1046,9 +1105,12 @@ int iris_batch_info(const iris_batch* B, long* info) {
   info[3] = B->master->K;
   info[4] = B->tile;
   info[5] = B->nitems;
-  if (B->tile == FUSED)
+  if (B->tile == FUSED) {
     for (const MarchCell& m : B->march[0]) info[5] += m.n;
-  const long in = B->tile == FUSED ? ((long)B->march[0].size() + MARCH_CELLS - 1) / MARCH_CELLS : 0;
+    for (const SlabCell& m : B->slab[0]) info[5] += m.n;
+  }
+  auto launches = [](size_t n) { return (long)(n + MARCH_CELLS - 1) / MARCH_CELLS; };
+  const long in = B->tile == FUSED ? launches(B->march[0].size()) + launches(B->slab[0].size()) : 0;
   info[6] = B->tile >= FLAT ? in + (B->nitems_in > 0) + (B->nitems > B->nitems_in) : 1;  // per E, H or fused pass
   info[7] = B->master->nslot;
   return IRIS_OK;

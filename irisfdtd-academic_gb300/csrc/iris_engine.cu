@@ -1991,7 +1991,7 @@ __global__ void __launch_bounds__(256) k_flux(const ACC* __restrict__ fd, long P
 // Fused E+H pass (FP32): one CTA per column tile and z chunk of the launch;
 // the tile column itself is fused_column (iris_fused.cuh).
 
-template <bool CEPS, bool UPML, typename IT>
+template <bool CEPS, bool UPML>
 __global__ void __launch_bounds__(FZ_X* FZ_Y, 2) k_fused(FusedArgs A) {
   __shared__ FusedSmem S;
   extern __shared__ __align__(16) unsigned char fz_dyn[];
@@ -1999,7 +1999,7 @@ __global__ void __launch_bounds__(FZ_X* FZ_Y, 2) k_fused(FusedArgs A) {
   const bool r0 = (int)blockIdx.z < A.nc0;
   const int z0 = r0 ? A.za0 + A.zc0 * (int)blockIdx.z : A.za1 + A.zc1 * ((int)blockIdx.z - A.nc0);
   const int z1 = min(z0 + (r0 ? A.zc0 : A.zc1) - 1, r0 ? A.zb0 : A.zb1);
-  fused_column<CEPS, UPML, IT>(A, S, U, blockIdx.x, blockIdx.y, z0, z1);
+  fused_column<CEPS, UPML>(A, S, U, blockIdx.x, blockIdx.y, z0, z1);
 }
 
 // Planes za..zb, outside the UPML slabs, by staged tiles (iris_march.cuh):
@@ -2008,6 +2008,25 @@ template <typename TL, bool CEPS> __global__ void __launch_bounds__(MR_T, 2) k_m
   extern __shared__ __align__(128) unsigned char mr_dyn[];
   const int z0 = za + zc * (int)blockIdx.z, z1 = min(z0 + zc - 1, zb);
   march_tile<TL, CEPS>(A, mr_dyn, blockIdx.x, blockIdx.y, z0, z1);
+}
+// The slabs, likewise: blockIdx.z < nc0 covers planes za0..zb0, the rest
+// za1..zb1.
+template <typename TL, bool CEPS>
+__global__ void __launch_bounds__(MS_T, 2) k_march_slab(MarchSlabArgs A, int za0, int zb0, int zc0, int nc0, int za1,
+                                                        int zb1, int zc1) {
+  extern __shared__ __align__(128) unsigned char mr_dyn[];
+  const bool r0 = (int)blockIdx.z < nc0;
+  const int z0 = r0 ? za0 + zc0 * (int)blockIdx.z : za1 + zc1 * ((int)blockIdx.z - nc0);
+  const int z1 = min(z0 + (r0 ? zc0 : zc1) - 1, r0 ? zb0 : zb1);
+  march_tile<TL, CEPS>(A.m, mr_dyn, blockIdx.x, blockIdx.y, z0, z1, A.d_new);
+}
+using SlabFn = void (*)(MarchSlabArgs, int, int, int, int, int, int, int);
+SlabFn slab_kernel(int id, bool cplx) {
+#define IRIS_SLAB_K(ID, W, R) \
+  if (id == ID) return cplx ? (SlabFn)k_march_slab<SlabTile<W, R>, true> : (SlabFn)k_march_slab<SlabTile<W, R>, false>;
+  IRIS_SLAB_SHAPES(IRIS_SLAB_K)
+#undef IRIS_SLAB_K
+  return nullptr;
 }
 using MarchFn = void (*)(MarchArgs, int, int, int);
 MarchFn march_kernel(int id, bool cplx) {
@@ -2250,28 +2269,28 @@ double fused_fill(int nx, int ny) {
 }
 
 // z chunks of planes za..zb for a launch of fused_column over `tiles` column
-// tiles: at least 48 planes each where the tiles fill the chip (each chunk
-// also reads the H plane below it and forms E' on the plane above it; measured
-// on GB300 against 16 planes: 512x512x1024 4.91 against 5.04 ms a pass), and
-// as few as 4 where they do not: a slab of 17 planes in one chunk is a chain
-// of 17 planes' latencies (64x64x512: 118 us a step, with 5 planes 90;
-// 128x128x128 111 and 87).
-// Appends (za, zb, planes per chunk, chunks) to r.
+// tiles: about 32 waves of two CTAs per SM, at least 48 planes each (each
+// chunk also reads the H plane below it and forms E' on the plane above it;
+// 512x512x1024 on GB300: 4.91 ms a pass, with 8 waves of at least 16 planes
+// 5.04).  Appends (za, zb, planes per chunk, chunks) to r.
 void fused_chunks(std::vector<int>& r, int za, int zb, long tiles) {
-  if (zb < za) return;
   const int len = zb - za + 1;
-  const long full = 2 * 152;
-  long nch = std::min<long>((32 * full + tiles - 1) / tiles, std::max(1, len / 48));
-  nch = std::max(nch, std::min<long>((full / 2 + tiles - 1) / tiles, len / 4));
+  const long nch = std::min<long>((32L * 152 * 2 + tiles - 1) / tiles, std::max(1, len / 48));
   const int zc = (int)((len + nch - 1) / nch);
   r.insert(r.end(), {za, zb, zc, (len + zc - 1) / zc});
 }
 
-// The march of planes (za, zb, zc, n) on the engine's stream.
-void launch_march(iris_engine* E, const std::vector<int>& r) {
+// The march of planes (za, zb, zc, n).
+void launch_march(iris_engine* E, const std::vector<int>& r, cudaStream_t st) {
   const MarchArgs a = march_args(E);
-  march_kernel(E->mshape.id, E->eps_complex)<<<dim3(a.tx, a.ty, r[3]), MR_T, E->mshape.smem, E->st>>>(a, r[0], r[1],
-                                                                                                     r[2]);
+  march_kernel(E->mshape.id, E->eps_complex)<<<dim3(a.tx, a.ty, r[3]), MR_T, E->mshape.smem, st>>>(a, r[0], r[1], r[2]);
+}
+// The slabs' (one or two ranges).
+void launch_slabs(iris_engine* E, const std::vector<int>& r, cudaStream_t st) {
+  const MarchSlabArgs a = march_slab_args(E);
+  const bool two = r.size() > 4;
+  slab_kernel(E->sshape.id, E->eps_complex)<<<dim3(a.m.tx, a.m.ty, r[3] + (two ? r[7] : 0)), MS_T, E->sshape.smem, st>>>(
+      a, r[0], r[1], r[2], r[3], two ? r[4] : 0, two ? r[5] : 0, two ? r[6] : 1);
 }
 
 // One fused step into the second buffers, swap, then TF/SF and the DFT
@@ -2293,24 +2312,20 @@ void fused_one(iris_engine* E, int it, int left, const int* itp, bool sampled) {
     for (int part = 1; part >= 0; --part) {
       const std::vector<int>& r = E->fzr[part];
       if (r.empty()) continue;
-      if (part == 0 && E->mshape.id >= 0) {
-        launch_march(E, r);
+      cudaStream_t st = part == 1 && both ? E->st2 : E->st;
+      if (E->mshape.id >= 0) {
+        if (part == 0) launch_march(E, r, st);
+        else launch_slabs(E, r, st);
         continue;
       }
       const FusedArgs a = fused_args(E, part);
       const dim3 grd(E->fgrd.x, E->fgrd.y, (unsigned)(r[3] + (r.size() > 4 ? r[7] : 0)));
       if (part == 0) {
-        if (E->eps_complex) k_fused<true, false, long><<<grd, E->fblk, 0, E->st>>>(a);
-        else k_fused<false, false, long><<<grd, E->fblk, 0, E->st>>>(a);
+        if (E->eps_complex) k_fused<true, false><<<grd, E->fblk, 0, st>>>(a);
+        else k_fused<false, false><<<grd, E->fblk, 0, st>>>(a);
       } else {
-        cudaStream_t s = both ? E->st2 : E->st;
-        if (E->fz_i32) {
-          if (E->eps_complex) k_fused<true, true, int><<<grd, E->fblk, FZ_UPML_SMEM, s>>>(a);
-          else k_fused<false, true, int><<<grd, E->fblk, FZ_UPML_SMEM, s>>>(a);
-        } else {
-          if (E->eps_complex) k_fused<true, true, long><<<grd, E->fblk, FZ_UPML_SMEM, s>>>(a);
-          else k_fused<false, true, long><<<grd, E->fblk, FZ_UPML_SMEM, s>>>(a);
-        }
+        if (E->eps_complex) k_fused<true, true><<<grd, E->fblk, FZ_UPML_SMEM, st>>>(a);
+        else k_fused<false, true><<<grd, E->fblk, FZ_UPML_SMEM, st>>>(a);
       }
     }
     if (both) {
@@ -3297,27 +3312,34 @@ int create_engine(const iris_params* pin, const double* fw, bool member, bool z_
     }
     // z chunks: planes pmlzi+1 .. pmlzf-2 (the last chunk's extra plane,
     // whose E' its H' needs, is then still outside the slabs) by the kernel
-    // without slab code, the slabs with the plane next to each by the other
+    // without slab code, the slabs with the plane next to each by the other;
+    // staged where 32-bit offsets reach
+    const bool staged = 3 * g.comp < (1L << 31);
+    if (staged) {
+      E->mshape = march_shape(p.nx, p.ny);
+      E->sshape = slab_shape(p.nx, p.ny);
+      for (bool c : {false, true})
+        if (cudaFuncSetAttribute((const void*)march_kernel(E->mshape.id, c), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)E->mshape.smem) != cudaSuccess ||
+            cudaFuncSetAttribute((const void*)slab_kernel(E->sshape.id, c), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)E->sshape.smem) != cudaSuccess)
+          return bail(fail(IRIS_ECUDA, "fused pass: shared memory configuration failed"));
+    }
     const long tiles = (long)((p.nx + FZ_OX - 1) / FZ_OX) * ((p.ny + FZ_OY - 1) / FZ_OY);
+    auto chunks = [&](int part, int za, int zb) {
+      if (zb < za) return;
+      if (!staged) return fused_chunks(E->fzr[part], za, zb, tiles);
+      const int len = zb - za + 1, zc = part == 0 ? march_chunk(len) : slab_chunk(len);
+      E->fzr[part].insert(E->fzr[part].end(), {za, zb, zc, (len + zc - 1) / zc});
+    };
     const int ia = p.pmlzi + 1, ib = p.pmlzf - 2;
     for (int part = 0; part < 2; ++part) E->fzr[part].clear();
     if (ib >= ia) {
-      // the staged march where its tiles fill and 32-bit offsets reach
-      if (3 * g.comp < (1L << 31)) {
-        E->mshape = march_shape(p.nx, p.ny);
-        const int zc = march_chunk(ib - ia + 1);
-        E->fzr[0] = {ia, ib, zc, (ib - ia + zc) / zc};
-        for (bool c : {false, true})
-          if (cudaFuncSetAttribute((const void*)march_kernel(E->mshape.id, c), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)E->mshape.smem) != cudaSuccess)
-            return bail(fail(IRIS_ECUDA, "fused pass: shared memory configuration failed"));
-      } else {
-        fused_chunks(E->fzr[0], ia, ib, tiles);
-      }
-      fused_chunks(E->fzr[1], 1, ia - 1, tiles);
-      fused_chunks(E->fzr[1], ib + 1, p.nz, tiles);
+      chunks(0, ia, ib);
+      chunks(1, 1, ia - 1);
+      chunks(1, ib + 1, p.nz);
     } else {
-      fused_chunks(E->fzr[1], 1, p.nz, tiles);
+      chunks(1, 1, p.nz);
     }
     E->fblk = dim3(FZ_X, FZ_Y, 1);
     int prio_lo = 0, prio_hi = 0;
@@ -3326,12 +3348,10 @@ int create_engine(const iris_params* pin, const double* fw, bool member, bool z_
         cudaEventCreateWithFlags(&E->fz_fork, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&E->fz_join, cudaEventDisableTiming) != cudaSuccess)
       return bail(fail(IRIS_ECUDA, "fused pass: stream creation failed"));
-    for (const void* kf : {(const void*)k_fused<false, true, long>, (const void*)k_fused<true, true, long>,
-                           (const void*)k_fused<false, true, int>, (const void*)k_fused<true, true, int>})
+    for (const void* kf : {(const void*)k_fused<false, true>, (const void*)k_fused<true, true>})
       if (cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FZ_UPML_SMEM) != cudaSuccess)
         return bail(fail(IRIS_ECUDA, "fused pass: shared memory configuration failed"));
     E->fgrd = dim3((p.nx + FZ_OX - 1) / FZ_OX, (p.ny + FZ_OY - 1) / FZ_OY, 1);
-    E->fz_i32 = 3 * E->g.comp < (1L << 31);
   }
   if (cudaMalloc(&E->d_err, sizeof(int)) != cudaSuccess) return bail(fail(IRIS_ENOMEM, "allocation failed"));
   cudaMemsetAsync(E->d_err, 0, sizeof(int), E->st);

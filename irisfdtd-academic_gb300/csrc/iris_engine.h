@@ -106,8 +106,7 @@ struct iris_engine {
   // the UPML slabs, [1] the slabs
   std::vector<int> fzr[2];
   dim3 fblk, fgrd;
-  iris::MarchShape mshape;  // tile shape of the staged pass of [0] (id < 0: not used)
-  bool fz_i32 = false;  // the fused pass's offsets fit int (3 x comp < 2^31)
+  iris::MarchShape mshape, sshape;  // tile shapes of the staged passes of [0], [1] (id < 0: not used)
   // the slab launch runs on st2, concurrently with the interior launch (they
   // write disjoint planes and read only the old state): fork / join events
   cudaStream_t st2 = nullptr;
@@ -224,6 +223,15 @@ inline MarchArgs march_args(const iris_engine* E) {
   a.h_new = (float2*)E->h2;
   a.tx = E->mshape.tx;
   a.ty = E->mshape.ty;
+  return a;
+}
+
+inline MarchSlabArgs march_slab_args(const iris_engine* E) {
+  MarchSlabArgs a{};
+  a.m = march_args(E);
+  a.m.tx = E->sshape.tx;
+  a.m.ty = E->sshape.ty;
+  for (int s = 0; s < 2; ++s) a.d_new[s] = (float2*)E->pml_d2[s];
   return a;
 }
 

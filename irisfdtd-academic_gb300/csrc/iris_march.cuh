@@ -54,6 +54,12 @@ struct MarchArgs {
   float2* h_new;
   int tx, ty;          // tiles of the plane
 };
+// The slabs' march: D is double buffered (image and overlap cells read the old
+// D of cells another CTA owns), B is its owner's and stays in place.
+struct MarchSlabArgs {
+  MarchArgs m;
+  float2* d_new[2];
+};
 
 __device__ __forceinline__ void march_cpa16(unsigned dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
@@ -62,31 +68,38 @@ __device__ __forceinline__ void march_cpa8(unsigned dst, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
 }
 
-template <int W_, int R_> struct MarchTile {
-  static constexpr int W = W_, R = R_, WT = W + 1, NC = (W + 1) * (R + 1);
+// T: threads of a CTA.  UPML: with the old D and B of its cells and the
+// coefficient rows in the ring.
+template <int W_, int R_, int T_ = MR_T, bool UPML_ = false> struct MarchTile {
+  static constexpr int W = W_, R = R_, T = T_, WT = W + 1, NC = (W + 1) * (R + 1);
+  static constexpr bool UPML = UPML_;
   static constexpr int BXH = (W + 4) / 2 * 2, BXE = (W + 2) / 2 * 2;  // columns of a box: x0-2 .., x0 ..
   static constexpr int HC = (R + 2) * BXH, EC = (R + 1) * BXE;        // elements of a component of a box
   static constexpr int HB = 3 * HC * 8, EB = 3 * EC * 8;              // bytes of a plane's box
   static constexpr int NI = W + R + 2;                                // image slots
-  static constexpr int SMEM = 4 * (HB + EB) + 4 * 2 * NI * 8;
+  static constexpr int UB = UPML ? 6 * T * 8 + 2 * NCOEF * 4 : 0;     // bytes of a plane's D, B and coefficients
+  static constexpr int SMEM = 4 * (HB + EB) + 4 * 2 * NI * 8 + 4 * UB;
   static constexpr int PH = 3 * HC / 2, PE = 3 * EC / 2;              // 16-byte pieces of a plane
-  static_assert(W % 2 == 0 && NC <= MR_T * MR_S && SMEM <= 112 * 1024, "tile shape");
+  static_assert(W % 2 == 0 && NC <= T * MR_S && SMEM <= 112 * 1024 && (!UPML || MR_S == 1), "tile shape");
 };
 
 // Planes z0..z1 of tile (bx, by): every thread of the CTA.  EDGE: the tile
 // touches a border of the plane.
 template <typename TL, bool CEPS, bool EDGE>
-__device__ __forceinline__ void march_column(const MarchArgs& A, unsigned char* smem, int bx, int by, int z0, int z1) {
+__device__ __forceinline__ void march_column(const MarchArgs& A, unsigned char* smem, int bx, int by, int z0, int z1,
+                                             float2* const* d_new = nullptr) {
   const FieldArgs<float>& a = A.f;
   const Geo& g = a.g;
   constexpr int HC = TL::HC, EC = TL::EC, BXH = TL::BXH, BXE = TL::BXE, NI = TL::NI;
-  constexpr int JH = (TL::PH + MR_T - 1) / MR_T, JE = (TL::PE + MR_T - 1) / MR_T;
+  constexpr int JH = (TL::PH + TL::T - 1) / TL::T, JE = (TL::PE + TL::T - 1) / TL::T;
+  constexpr bool UPML = TL::UPML;
   const int t = threadIdx.x;
   const int x0 = 1 + bx * TL::W, y0 = 1 + by * TL::R;
   unsigned char* const sh = smem;                              // 4 planes of H
   unsigned char* const se = smem + 4 * TL::HB;                 // 4 planes of E, then E'
   float2* const si = (float2*)(smem + 4 * (TL::HB + TL::EB));  // the images' H at x = 0 [row], y = 0 [R+1+col]: [4][2][NI]
-  if (!bc_ok(z0 >= 2 && z1 + 1 <= g.nz && z0 <= z1 + 1, BC_FUSED_CELL, ((long)z0 << 32) | (unsigned)z1)) return;
+  unsigned char* const su = smem + 4 * (TL::HB + TL::EB) + 4 * 2 * NI * 8;  // UPML: [4][D, B: [6][T]; E, H rows]
+  if (!bc_ok(z0 >= (UPML ? 1 : 2) && z1 + (UPML ? 0 : 1) <= g.nz && z0 <= z1 + 1, BC_FUSED_CELL, ((long)z0 << 32) | (unsigned)z1)) return;
   const float2* E = a.e;
   const float2* H = a.h;
   const int pl = (int)g.plane, pt = (int)g.pitch, cp = (int)g.comp;
@@ -100,8 +113,8 @@ __device__ __forceinline__ void march_column(const MarchArgs& A, unsigned char* 
   cx<float> ev[MR_S][3];  // E' of the plane below
 #pragma unroll
   for (int s = 0; s < MR_S; ++s) {
-    const int c = t + s * MR_T, row = c / TL::WT, col = c - row * TL::WT, x = x0 + col, y = y0 + row;
-    act[s] = (s * MR_T + MR_T <= TL::NC || c < TL::NC) && (!EDGE || (x <= g.nx + 1 && y <= g.ny + 1));
+    const int c = t + s * TL::T, row = c / TL::WT, col = c - row * TL::WT, x = x0 + col, y = y0 + row;
+    act[s] = (s * TL::T + TL::T <= TL::NC || c < TL::NC) && (!EDGE || (x <= g.nx + 1 && y <= g.ny + 1));
     own[s] = act[s] && col < TL::W && row < TL::R && (!EDGE || (x <= g.nx && y <= g.ny));
     ih[s] = (row + 1) * BXH + col + 2;
     ie[s] = row * BXE + col;
@@ -120,7 +133,7 @@ __device__ __forceinline__ void march_column(const MarchArgs& A, unsigned char* 
   }
   // this thread's 16-byte pieces of the boxes: storage offset on plane 0 (-1:
   // none, past the storage rows, which only cells that are not computed would
-  // read); piece t + j MR_T lies (t + j MR_T) 16 bytes into a plane of the
+  // read); piece t + j TL::T lies (t + j TL::T) 16 bytes into a plane of the
   // ring.  EDGE: a piece at x = nx+1 comes from x = 1; where it begins at nx,
   // its second half does (bit j of a mask; the row starts at go - xi).
   int gh[JH], ge[JE];
@@ -142,13 +155,13 @@ __device__ __forceinline__ void march_column(const MarchArgs& A, unsigned char* 
 #pragma unroll
   for (int j = 0; j < JH; ++j) {
     bool sp;
-    gh[j] = piece(t + j * MR_T, TL::PH, BXH, TL::R + 2, x0 - 2, y0 - 1, sp);
+    gh[j] = piece(t + j * TL::T, TL::PH, BXH, TL::R + 2, x0 - 2, y0 - 1, sp);
     if (sp) mh |= 1u << j;
   }
 #pragma unroll
   for (int j = 0; j < JE; ++j) {
     bool sp;
-    ge[j] = piece(t + j * MR_T, TL::PE, BXE, TL::R + 1, x0, y0, sp);
+    ge[j] = piece(t + j * TL::T, TL::PE, BXE, TL::R + 1, x0, y0, sp);
     if (sp) me |= 1u << j;
   }
   const unsigned uh = smem_u32(sh) + 16u * t, ue = smem_u32(se) + 16u * t;
@@ -160,26 +173,56 @@ __device__ __forceinline__ void march_column(const MarchArgs& A, unsigned char* 
       march_cpa16(dst, src);
     }
   };
+  // UPML: this thread's cell within a plane of D and B
+  const int px = EDGE && (ed[0] & 16) ? 1 : x0 + t % TL::WT, py = EDGE && (ed[0] & 32) ? 1 : y0 + t / TL::WT;
+  auto in_slab = [&](int z) { return z <= a.pmlzi || z >= a.pmlzf; };
   // everything of plane p into its ring place p & 3: one commit group a plane
   auto ahead = [&](int p) {
     if (p <= z1 + 1) {
-      const int zo = p * pl;
+      const int zo = (UPML && p == g.nz + 1 ? 1 : p) * pl;
+      if (UPML && p >= z0) {
+        // the old D of this thread's E' cell on the plane, the B of its own
+        // cell on the plane below, and both planes' coefficient rows
+        unsigned char* const u = su + (p & 3) * TL::UB;
+        const int ze = p == g.nz + 1 ? 1 : p, zb = p - 1;
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const int z = q == 0 ? ze : zb;
+          if (!in_slab(z) || (q == 1 && zb < z0)) continue;
+          const int slab = z <= a.pmlzi ? 0 : 1, zr = slab == 0 ? z - 1 : z - a.pmlzf;
+          if (q == 0 ? act[0] : own[0]) {
+            const long pi = ((long)zr * g.ny + (py - 1)) * (long)g.nx + (px - 1);
+            const float2* src = (q == 0 ? a.pml_d[slab] : a.pml_b[slab]) + pi;
+            if (bc_ok(pi >= 0 && pi < a.pcomp[slab], BC_FUSED_SLAB, pi))
+#pragma unroll
+              for (int k = 0; k < 3; ++k)
+                march_cpa8(smem_u32(u) + 8u * ((3 * q + k) * TL::T + t), src + k * a.pcomp[slab]);
+          }
+          if ((t >> 5) == q && (t & 31) < NCOEF) {
+            const float* src = a.coef + NCOEF * (slab == 0 ? z - 1 : a.pmlzi + z - a.pmlzf) + (t & 31);
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(u) + 48u * TL::T +
+                                                                          4u * (q * NCOEF + (t & 31))),
+                         "l"(src)
+                         : "memory");
+          }
+        }
+      }
       const unsigned dh = uh + (unsigned)((p & 3) * TL::HB), de = ue + (unsigned)((p & 3) * TL::EB);
 #pragma unroll
       for (int j = 0; j < JH; ++j)
-        if ((!EDGE && (j + 1) * MR_T <= TL::PH) || gh[j] >= 0)
-          copy(dh + 16u * MR_T * j, H + (gh[j] + zo), (mh >> j) & 1u);
+        if ((!EDGE && (j + 1) * TL::T <= TL::PH) || gh[j] >= 0)
+          copy(dh + 16u * TL::T * j, H + (gh[j] + zo), (mh >> j) & 1u);
       if (p >= z0) {
 #pragma unroll
         for (int j = 0; j < JE; ++j)
-          if ((!EDGE && (j + 1) * MR_T <= TL::PE) || ge[j] >= 0)
-            copy(de + 16u * MR_T * j, E + (ge[j] + zo), (me >> j) & 1u);
+          if ((!EDGE && (j + 1) * TL::T <= TL::PE) || ge[j] >= 0)
+            copy(de + 16u * TL::T * j, E + (ge[j] + zo), (me >> j) & 1u);
         if (EDGE) {
 #pragma unroll
           for (int s = 0; s < MR_S; ++s) {
             if (!act[s] || !(ed[s] & 48)) continue;
             const unsigned d = smem_u32(si + (p & 3) * 2 * NI);
-            const int c = t + s * MR_T, row = c / TL::WT, col = c - row * TL::WT, q = zo + oc[s];
+            const int c = t + s * TL::T, row = c / TL::WT, col = c - row * TL::WT, q = zo + oc[s];
             if (ed[s] & 16) {
               march_cpa8(d + 8u * row, H + (cp + q - 1));
               march_cpa8(d + 8u * (NI + row), H + (2 * cp + q - 1));
@@ -195,6 +238,7 @@ __device__ __forceinline__ void march_column(const MarchArgs& A, unsigned char* 
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
   auto eps_of = [&](int p) {  // the structure's eps_inv of plane p, loaded one plane ahead
+    if (UPML && p == g.nz + 1) p = 1;
     if (p >= a.hi && p <= a.hf) {
 #pragma unroll
       for (int s = 0; s < MR_S; ++s)
@@ -220,8 +264,9 @@ __device__ __forceinline__ void march_column(const MarchArgs& A, unsigned char* 
     const float2* hm = (const float2*)(sh + ((z + 3) & 3) * TL::HB);  // plane z-1
     float2* ez = (float2*)(se + (z & 3) * TL::EB);
     const float2* em = (const float2*)(se + ((z + 3) & 3) * TL::EB);  // E' of plane z-1
-    const bool mat = z >= a.hi && z <= a.hf;
-    const float mz = z < a.hi ? a.m1 : a.m3;
+    const int zc = UPML && z == g.nz + 1 ? 1 : z;
+    const bool mat = zc >= a.hi && zc <= a.hf;
+    const float mz = zc < a.hi ? a.m1 : a.m3;
 #pragma unroll
     for (int s = 0; s < MR_S; ++s) {
       if (!act[s]) continue;
@@ -241,7 +286,7 @@ __device__ __forceinline__ void march_column(const MarchArgs& A, unsigned char* 
         for (int k = 0; k < 3; ++k) en[k] = get(ez + ie[s] + k * EC);
       }
       if (EDGE && (ed[s] & 48)) {
-        const int c = t + s * MR_T, row = c / TL::WT, col = c - row * TL::WT;
+        const int c = t + s * TL::T, row = c / TL::WT, col = c - row * TL::WT;
         const float2* p = si + (z & 3) * 2 * NI;
         if (ed[s] & 16) {
           hx1 = get(p + row);
@@ -252,10 +297,19 @@ __device__ __forceinline__ void march_column(const MarchArgs& A, unsigned char* 
           hy2 = get(p + NI + TL::R + 1 + col);
         }
       }
+      if (UPML && z == g.nz + 1) {  // the image of plane 1, above H's ghost plane
+        hz0 = ld<float>(H + oc[s]);
+        hz1 = ld<float>(H + (cp + oc[s]));
+      }
       cu[0] = cadd(csub(csub(h2, hy2), h1), hz1);
       cu[1] = cadd(csub(csub(h0, hz0), h2), hx2);
       cu[2] = cadd(csub(csub(h1, hx1), h0), hy0);
-      if (CEPS && mat) {
+      if (UPML && in_slab(zc)) {
+        const float2* u = (const float2*)(su + (z & 3) * TL::UB);
+        const cx<float> dv[3] = {get(u + t), get(u + TL::T + t), get(u + 2 * TL::T + t)};
+        e_apply<float, CEPS, 7, !CEPS, true>(a, own[s] && z <= z1 ? d_new : nullptr, px, py, zc, cu, en, 0.f, dv,
+                                             (const float*)(u + 6 * TL::T));
+      } else if (CEPS && mat) {
 #pragma unroll
         for (int k = 0; k < 3; ++k) en[k] = cadd(en[k], cmul(epc[CEPS ? s : 0], cu[k]));
       } else {
@@ -269,6 +323,10 @@ __device__ __forceinline__ void march_column(const MarchArgs& A, unsigned char* 
         if (ed[s] & 32) ph = cmul(ph, a.pyp);
 #pragma unroll
         for (int k = 0; k < 3; ++k) en[k] = cmul(ph, en[k]);
+      }
+      if (UPML && z == g.nz + 1) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) en[k] = cmul(a.pzp, en[k]);
       }
 #pragma unroll
       for (int k = 0; k < 3; ++k) ez[ie[s] + k * EC] = make_float2(en[k].re, en[k].im);
@@ -287,10 +345,25 @@ __device__ __forceinline__ void march_column(const MarchArgs& A, unsigned char* 
           hn[0] = hz0;
           hn[1] = hz1;
           hn[2] = get(hm + ih[s] + 2 * HC);
-          h_update<float, false>(a, 1, 1, 1, ev[s], xp, yp, zp, hn);
+          if (UPML) {
+            hn[0] = get(hm + ih[s]);
+            hn[1] = get(hm + ih[s] + HC);
+            const float2* u = (const float2*)(su + (z & 3) * TL::UB);
+            const cx<float> bv[3] = {get(u + 3 * TL::T + t), get(u + 4 * TL::T + t), get(u + 5 * TL::T + t)};
+            h_update<float, true>(a, px, py, z - 1, ev[s], xp, yp, zp, hn, bv, (const float*)(u + 6 * TL::T) + NCOEF);
+          } else {
+            h_update<float, false>(a, 1, 1, 1, ev[s], xp, yp, zp, hn);
+          }
           const int j = i - pl;
 #pragma unroll
           for (int k = 0; k < 3; ++k) st<float>(A.h_new + (k * cp + j), hn[k]);
+          if (UPML && z - 1 == g.nz) {
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+              st<float>(A.e_new + (k * cp + j - g.nz * pl), cmul(a.pzm, ev[s][k]));
+              st<float>(A.h_new + (k * cp + j - g.nz * pl), cmul(a.pzm, hn[k]));
+            }
+          }
           if (EDGE && (ed[s] & 1)) {
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
@@ -309,6 +382,10 @@ __device__ __forceinline__ void march_column(const MarchArgs& A, unsigned char* 
         if (z <= z1) {
 #pragma unroll
           for (int k = 0; k < 3; ++k) st<float>(A.e_new + (k * cp + i), en[k]);
+          if (UPML && z == 1) {
+#pragma unroll
+            for (int k = 0; k < 3; ++k) st<float>(A.e_new + (k * cp + i + g.nz * pl), cmul(a.pzp, en[k]));
+          }
           if (EDGE && (ed[s] & 4)) {
 #pragma unroll
             for (int k = 0; k < 3; ++k) st<float>(A.e_new + (k * cp + i + g.nx), cmul(a.pxp, en[k]));
@@ -333,11 +410,12 @@ __device__ __forceinline__ void march_column(const MarchArgs& A, unsigned char* 
 }
 
 template <typename TL, bool CEPS>
-__device__ __forceinline__ void march_tile(const MarchArgs& A, unsigned char* smem, int bx, int by, int z0, int z1) {
+__device__ __forceinline__ void march_tile(const MarchArgs& A, unsigned char* smem, int bx, int by, int z0, int z1,
+                                           float2* const* d_new = nullptr) {
   if (bx == 0 || by == 0 || bx == A.tx - 1 || by == A.ty - 1)
-    march_column<TL, CEPS, true>(A, smem, bx, by, z0, z1);
+    march_column<TL, CEPS, true>(A, smem, bx, by, z0, z1, d_new);
   else
-    march_column<TL, CEPS, false>(A, smem, bx, by, z0, z1);
+    march_column<TL, CEPS, false>(A, smem, bx, by, z0, z1, d_new);
 }
 
 // The tile shapes, and the one taken for an nx x ny plane: the fewest bytes of
@@ -350,6 +428,17 @@ __device__ __forceinline__ void march_tile(const MarchArgs& A, unsigned char* sm
 #define IRIS_MARCH_SMEM(ID, W, R) MarchTile<W, R>::SMEM,
 constexpr int MARCH_MAX_SMEM = std::max({IRIS_MARCH_SHAPES(IRIS_MARCH_SMEM) 0});
 #undef IRIS_MARCH_SMEM
+// The slabs' march: the same column with the old D and B of its cells and the
+// coefficients in the ring, tiles half the size (two CTAs of 256 threads an SM).
+// Of a pass of 512x512x256 with slabs of 17 planes fused_column took 480 us at
+// 38 % of the copy bandwidth, and the pass 1420 us; it takes 1321 so, 256x256x512
+// 625 instead of 662, 256x256x96 159 instead of 167.
+#define IRIS_SLAB_SHAPES(F) F(0, 32, 6) F(1, 24, 9) F(2, 16, 14) F(3, 40, 5)
+constexpr int MS_T = 256;
+template <int W, int R> using SlabTile = MarchTile<W, R, MS_T, true>;
+#define IRIS_SLAB_SMEM(ID, W, R) SlabTile<W, R>::SMEM,
+constexpr int SLAB_MAX_SMEM = std::max({IRIS_SLAB_SHAPES(IRIS_SLAB_SMEM) 0});
+#undef IRIS_SLAB_SMEM
 struct MarchShape {
   int id = -1, tx = 0, ty = 0;  // id < 0: none
   size_t smem = 0;
@@ -371,9 +460,33 @@ inline MarchShape march_shape(int nx, int ny) {
 #undef IRIS_MARCH_TRY
   return best;
 }
+inline MarchShape slab_shape(int nx, int ny) {
+  MarchShape best;
+  double cost = 1e300;
+#define IRIS_SLAB_TRY(ID, W, R)                                         \
+  {                                                                     \
+    const int tx = (nx + W - 1) / W, ty = (ny + R - 1) / R;             \
+    const double c = (double)tx * ty * (W + 24) * (R + 1.5);            \
+    if (c < cost) {                                                     \
+      cost = c;                                                         \
+      best.id = ID, best.tx = tx, best.ty = ty;                         \
+      best.smem = SlabTile<W, R>::SMEM;                                 \
+    }                                                                   \
+  }
+  IRIS_SLAB_SHAPES(IRIS_SLAB_TRY)
+#undef IRIS_SLAB_TRY
+  return best;
+}
 // Planes of a z chunk of len planes: MR_CHUNK to 2 MR_CHUNK - 1, or len.
 inline int march_chunk(int len) {
   const int n = std::max(1, len / MR_CHUNK);
+  return (len + n - 1) / n;
+}
+
+// The same in the slabs: 12 to 23, or len (512x512x256, slabs of 17 planes, a
+// pass: 1359 us in chunks of 5 planes, 1334 of 9, 1321 of 17; 256x256x96 163, 160, 159).
+inline int slab_chunk(int len) {
+  const int n = std::max(1, len / 12);
   return (len + n - 1) / n;
 }
 

@@ -22,8 +22,7 @@ CASES = [(32, 14, 13, False), (33, 15, 14, True), (96, 42, 28, False), (24, 19, 
 
 
 @pytest.mark.parametrize("nx,ny,planes,lossy", CASES)
-def test_march_equals_split(iris, tmp_path, nx, ny, planes, lossy):
-    pml = 4
+def test_march_equals_split(iris, tmp_path, nx, ny, planes, lossy, pml=4):
     nz = planes + 2 * pml + 1  # the march takes planes pml + 1 .. nz - 1 - pml
     hi, dh = max(pml + 2, nz // 2 - 3), max(1, min(6, planes - 3))
     w = cfg.Workload("march", nx, ny, nz, pml, nz + 1 - pml, hi, dh, 2.25, 0, pml + 1,
@@ -81,3 +80,13 @@ def test_march_batch_equals_engines(iris, tmp_path):
         assert np.any(interior(b.get_field(c, iris.E), p))
         e.close()
     b.close()
+
+
+@pytest.mark.parametrize("nx,ny,pml,planes,lossy", [(32, 6, 25, 2, False), (33, 7, 13, 6, True), (96, 18, 12, 9, False),
+                                                    (24, 9, 24, 3, False), (25, 10, 11, 5, True), (16, 14, 48, 4, False),
+                                                    (17, 15, 23, 7, False), (40, 5, 12, 3, True), (121, 16, 30, 2, False),
+                                                    (1, 1, 37, 5, False)])
+def test_slab_march_equals_split(iris, tmp_path, nx, ny, pml, planes, lossy):
+    """The UPML slabs at the edges of their tile shapes (32x6, 24x9, 16x14 and
+    40x5) and chunks (12 to 23 planes)."""
+    test_march_equals_split(iris, tmp_path, nx, ny, planes, lossy, pml)
