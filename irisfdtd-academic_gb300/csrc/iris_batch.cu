@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(256) k_batch_gather(const FieldArgs<T>* __rest
   if (blockIdx.x * (unsigned)GATHER_BLOCK >= (unsigned)b.s.nu * (unsigned)b.s.nv) return;
   const FieldArgs<T>& a = args[b.cell];
   const typename V2<T>::t* src = b.s.field < 3 ? a.e + b.s.field * a.g.comp : a.h + (b.s.field - 3) * a.g.comp;
-  gather_run<T>(b.s, src, slot, a.g.comp, np);
+  gather_run<T>(b.s, src, slot, a.g.comp, np, blockIdx.x, threadIdx.x);
 }
 
 }  // namespace

@@ -685,10 +685,11 @@ constexpr int GATHER_PER = 4, GATHER_BLOCK = 256 * GATHER_PER;
 // by the bounds-check build).
 template <typename T>
 __device__ __forceinline__ void gather_run(const Seg& sg, const typename V2<T>::t* __restrict__ src,
-                                           typename V2<T>::t* __restrict__ slot, long comp, long np) {
+                                           typename V2<T>::t* __restrict__ slot, long comp, long np, unsigned block,
+                                           unsigned tid) {
   using V = typename V2<T>::t;
   const unsigned n = (unsigned)sg.nu * (unsigned)sg.nv, nu = (unsigned)sg.nu;
-  const unsigned L0 = blockIdx.x * (unsigned)GATHER_BLOCK + threadIdx.x;
+  const unsigned L0 = block * (unsigned)GATHER_BLOCK + tid;
   V val[GATHER_PER];
 #pragma unroll
   for (int j = 0; j < GATHER_PER; ++j) {

@@ -417,7 +417,29 @@ __global__ void __launch_bounds__(256) k_dft_gather(const typename V2<T>::t* __r
   if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) tk[islot] = tp ? *tp + t : t;
   const Seg sg = segs[blockIdx.y];
   const typename V2<T>::t* src = sg.field < 3 ? e + sg.field * comp : h + (sg.field - 3) * comp;
-  gather_run<T>(sg, src, slot, comp, np);
+  gather_run<T>(sg, src, slot, comp, np, blockIdx.x, threadIdx.x);
+}
+
+// Both in one launch, where no sample point lies on a corrected plane: the
+// first nt CTAs (tx across) correct, the others (gx a run) sample.  Each is a
+// few microseconds of latency after a launch gap as long: 160x160x512, 16.7
+// us a step apart, 9.2 together.
+template <typename T>
+__global__ void __launch_bounds__(256) k_tfsf_gather(typename V2<T>::t* e, typename V2<T>::t* h, Geo g, SrcArgs s,
+                                                     const TfsfVal<T>* __restrict__ row, unsigned nt, unsigned tx,
+                                                     const Seg* __restrict__ segs, unsigned gx,
+                                                     typename V2<T>::t* __restrict__ slot, int* tk, int islot, int t,
+                                                     const int* tp, long np) {
+  const unsigned b = blockIdx.x, tid = threadIdx.x;
+  if (b < nt) {
+    const int ix = (int)(b % tx * 64 + (tid & 63)), iy = (int)(b / tx * 4 + tid / 64);
+    if (ix <= s.nx + 1 && iy <= s.ny + 1) tfsf_apply<T>(e, h, g, s, ix, iy, row[ix]);
+    return;
+  }
+  if (b == nt && tid == 0) tk[islot] = tp ? *tp + t : t;
+  const Seg sg = segs[(b - nt) / gx];
+  const typename V2<T>::t* src = sg.field < 3 ? e + sg.field * g.comp : h + (sg.field - 3) * g.comp;
+  gather_run<T>(sg, src, slot, g.comp, np, (b - nt) % gx, tid);
 }
 
 // FP32 mode accumulators: each complex value of fdata is a compensated
@@ -2217,23 +2239,47 @@ template <typename T> void tfsf_table(iris_engine* E, int it, int n, const int* 
                                                                               (TfsfVal<T>*)E->d_tfv);
 }
 
+// Whether no DFT sample point lies on a plane the TF/SF corrections write
+// (E at iz_min, H at iz_min-1 in variant 1 and at iz_min in variant 2): then
+// corrections and sample share a launch, or k_tiny's TF/SF phase.
+bool sample_merges(const iris_engine* E) {
+  const int zm = E->src.iz_min;
+  const int zh = E->src.variant == 1 ? zm - 1 : zm;
+  for (const Seg& sg : E->segs) {
+    long lo = sg.src, hi = sg.src;
+    for (int cu = 0; cu < 2; ++cu)
+      for (int cv = 0; cv < 2; ++cv) {
+        const long q = sg.src + (cu ? (long)(sg.nu - 1) * sg.su : 0) + (cv ? (long)(sg.nv - 1) * sg.sv : 0);
+        lo = std::min(lo, q);
+        hi = std::max(hi, q);
+      }
+    const long z0 = lo / E->g.plane, z1 = hi / E->g.plane;
+    const int zc = sg.field < 3 ? zm : zh;
+    if (zc >= z0 && zc <= z1) return false;
+  }
+  return true;
+}
+
 // Step it's corrections; left: the steps the caller goes on to take, it
 // included.  The table is evaluated for as many of them as it holds whenever
 // the step lies outside the steps it covers (tf_at .. tf_end, reset by every
 // call that steps).
-template <typename T> void launch_tfsf(iris_engine* E, int it, int left, const int* itp = nullptr) {
-  if (E->src.variant == 0) return;
-  KTimer tm(E, IRIS_KC_TFSF);
-  using V = typename V2<T>::t;
+template <typename T> const TfsfVal<T>* tfsf_row(iris_engine* E, int it, int left, const int* itp) {
   if (it < E->tf_at || it >= E->tf_end) {
     const int n = std::max(1, std::min(left, E->tfv_cap));
     tfsf_table<T>(E, it, n, itp);
     E->tf_at = it;
     E->tf_end = it + n;
   }
+  return (const TfsfVal<T>*)E->d_tfv + (long)(it - E->tf_at) * (E->p.nx + 2);
+}
+template <typename T> void launch_tfsf(iris_engine* E, int it, int left, const int* itp = nullptr) {
+  if (E->src.variant == 0) return;
+  KTimer tm(E, IRIS_KC_TFSF);
+  using V = typename V2<T>::t;
+  const TfsfVal<T>* row = tfsf_row<T>(E, it, left, itp);
   const dim3 grd((unsigned)((E->p.nx + 2 + 63) / 64), (unsigned)((E->p.ny + 2 + 3) / 4));
-  k_tfsf<T><<<grd, dim3(64, 4), 0, E->st>>>((V*)E->e, (V*)E->h, E->g, E->src,
-                                            (const TfsfVal<T>*)E->d_tfv + (long)(it - E->tf_at) * (E->p.nx + 2));
+  k_tfsf<T><<<grd, dim3(64, 4), 0, E->st>>>((V*)E->e, (V*)E->h, E->g, E->src, row);
 }
 
 template <typename T> void dft_sample(iris_engine* E, int t, const int* tp = nullptr) {
@@ -2245,6 +2291,28 @@ template <typename T> void dft_sample(iris_engine* E, int t, const int* tp = nul
   dim3 grid((unsigned)((E->max_seg + GATHER_BLOCK - 1) / GATHER_BLOCK), (unsigned)E->segs.size());
   k_dft_gather<T><<<grid, 256, 0, E->st>>>((const V*)E->e, (const V*)E->h, E->g.comp, E->d_segs, slot, E->d_tk,
                                           E->nslot, t, tp, E->P);
+  }
+  if (++E->nslot == E->K) dft_flush(E);
+}
+
+// Step it's corrections and, when it is sampled, its DFT sample: in one
+// launch where they touch different planes (timed as the sample).
+template <typename T> void finish_step(iris_engine* E, int it, int left, const int* itp, bool sampled) {
+  const int t = it + 1 - E->p.to_fourier;
+  if (!sampled || E->P == 0 || E->src.variant == 0 || !E->merge) {
+    launch_tfsf<T>(E, it, left, itp);
+    if (sampled) dft_sample<T>(E, t, itp);
+    return;
+  }
+  using V = typename V2<T>::t;
+  {
+    KTimer tm(E, IRIS_KC_GATHER);
+    const TfsfVal<T>* row = tfsf_row<T>(E, it, left, itp);
+    const unsigned tx = (unsigned)((E->p.nx + 2 + 63) / 64), nt = tx * (unsigned)((E->p.ny + 2 + 3) / 4);
+    const unsigned gx = (unsigned)((E->max_seg + GATHER_BLOCK - 1) / GATHER_BLOCK);
+    k_tfsf_gather<T><<<nt + gx * (unsigned)E->segs.size(), 256, 0, E->st>>>(
+        (V*)E->e, (V*)E->h, E->g, E->src, row, nt, tx, E->d_segs, gx, (V*)E->S + (long)E->nslot * E->P, E->d_tk,
+        E->nslot, t, itp, E->P);
   }
   if (++E->nslot == E->K) dft_flush(E);
 }
@@ -2336,8 +2404,7 @@ void fused_one(iris_engine* E, int it, int left, const int* itp, bool sampled) {
   std::swap(E->e, E->e2);
   std::swap(E->h, E->h2);
   for (int s = 0; s < 2; ++s) std::swap(E->pml_d[s], E->pml_d2[s]);
-  launch_tfsf<float>(E, it, left, itp);
-  if (sampled) dft_sample<float>(E, it + 1 - E->p.to_fourier, itp);
+  finish_step<float>(E, it, left, itp, sampled);
 }
 
 int step_fused(iris_engine* E, int it0, int n) {
@@ -2371,8 +2438,7 @@ template <typename T> int step_t(iris_engine* E, int it0, int n) {
         for (int j = 0; j < E->K; ++j) {
           launch_e<T>(E);
           launch_h<T>(E);
-          launch_tfsf<T>(E, j, E->K - j, E->d_it);
-          dft_sample<T>(E, j + 1 - p.to_fourier, E->d_it);
+          finish_step<T>(E, j, E->K - j, E->d_it, true);
         }
       });
       E->tf_end = 0;
@@ -2382,33 +2448,11 @@ template <typename T> int step_t(iris_engine* E, int it0, int n) {
     }
     launch_e<T>(E);
     launch_h<T>(E);
-    launch_tfsf<T>(E, it, it0 + n - it);
-    if (it >= p.to_fourier && it % p.sample_fourier == 0) dft_sample<T>(E, it + 1 - p.to_fourier);
+    finish_step<T>(E, it, it0 + n - it, nullptr, it >= p.to_fourier && it % p.sample_fourier == 0);
     ++it;
   }
   CK(cudaGetLastError());
   return IRIS_OK;
-}
-
-// Whether no DFT sample point lies on a plane the TF/SF corrections write
-// (E at iz_min, H at iz_min-1 in variant 1 and at iz_min in variant 2): then
-// k_tiny samples in the TF/SF phase.
-static bool tiny_sample_merges(const iris_engine* E) {
-  const int zm = E->src.iz_min;
-  const int zh = E->src.variant == 1 ? zm - 1 : zm;
-  for (const Seg& sg : E->segs) {
-    long lo = sg.src, hi = sg.src;
-    for (int cu = 0; cu < 2; ++cu)
-      for (int cv = 0; cv < 2; ++cv) {
-        const long q = sg.src + (cu ? (long)(sg.nu - 1) * sg.su : 0) + (cv ? (long)(sg.nv - 1) * sg.sv : 0);
-        lo = std::min(lo, q);
-        hi = std::max(hi, q);
-      }
-    const long z0 = lo / E->g.plane, z1 = hi / E->g.plane;
-    const int zc = sg.field < 3 ? zm : zh;
-    if (zc >= z0 && zc <= z1) return false;
-  }
-  return true;
 }
 
 // The kernel of a resident engine.
@@ -2620,7 +2664,7 @@ int res_samples(iris_engine* E) {
 template <typename T> int step_persist(iris_engine* E, int it0, int n) {
   const iris_params& p = E->p;
   const int cap = E->src.variant != 0 ? E->tfv_cap : 1024;
-  const bool merged = !E->res && tiny_sample_merges(E);
+  const bool merged = !E->res && E->merge;
   if (E->res && !E->d_rsamp)
     if (int rc = res_samples(E)) return rc;
   if (!E->res && E->P > 0 && !E->d_sidx) {
@@ -3147,13 +3191,11 @@ void one_step(iris_engine* E, int it, int left, bool dft) {
   } else if (E->prec == IRIS_FP64) {
     launch_e<double>(E);
     launch_h<double>(E);
-    launch_tfsf<double>(E, it, left);
-    if (sampled) dft_sample<double>(E, it + 1 - p.to_fourier);
+    finish_step<double>(E, it, left, nullptr, sampled);
   } else {
     launch_e<float>(E);
     launch_h<float>(E);
-    launch_tfsf<float>(E, it, left);
-    if (sampled) dft_sample<float>(E, it + 1 - p.to_fourier);
+    finish_step<float>(E, it, left, nullptr, sampled);
   }
 }
 
@@ -3368,6 +3410,7 @@ int create_engine(const iris_params* pin, const double* fw, bool member, bool z_
   if (rc) return bail(rc);
   rc = build_dft(E);
   if (rc) return bail(rc);
+  E->merge = sample_merges(E);
   if (cudaStreamSynchronize(E->st) != cudaSuccess) return bail(fail(IRIS_ECUDA, "initialisation failed"));
   *out = E;
   return IRIS_OK;

@@ -66,6 +66,7 @@ struct iris_engine {
   iris::FaceMap fm[2][3];
   long P = 0;
   int K = 0, nslot = 0;
+  bool merge = false;  // the sample and the TF/SF corrections touch different planes
   std::vector<iris::Seg> segs;
   long max_seg = 0;
   iris::Seg* d_segs = nullptr;
