@@ -32,7 +32,10 @@ using namespace iris;
 //                   then Ebar <- al Ebar, Dbar <- a Dbar + g_e Ebar
 // Each "then" part touches one cell of a field whose neighbours the same
 // kernel still reads, so it is deferred to the next kernel, which reads only
-// its own cell of that field: both kernels update in place.
+// its own cell of that field: both kernels update in place.  In FP32 the planes
+// outside the slabs take both passes in one (iris_march.cuh), into second
+// buffers of E and H; the kernels here then do the slabs and the plane next to
+// each, from the old buffers into the new.
 // dL/d eps_inv(c) = sum_n Re <Ebar'_n(c), C_n(c)>, Ebar'_n the adjoint of the
 // E pass output of step n, C_n the forward curl of H that pass used.
 
@@ -52,8 +55,11 @@ struct Design {
 
 template <typename T> struct AdjArgs {
   FieldArgs<T> f;                // adjoint state; coef = adjoint rows, eps_r = forward material
-  int z0;                        // first plane of the launch (blockIdx.z counts from it)
-  int z1;                        // last plane of the launch
+  int z0, z1;                    // planes of the launch (blockIdx.z counts from z0): z0 .. z1,
+  int z2, z3;                    // then z2 .. z3 (none when z3 < z2)
+  typename V2<T>::t* eo;         // where the new E and H go (in place: f.e, f.h)
+  typename V2<T>::t* ho;
+  int images;                    // also store H's images at x = 0 and y = 0 (the march reads them)
   Design d;
   const typename V2<T>::t* rec;  // forward curl of H at the design cells for this step, [3][n]
   double* grad;                  // dL/d eps_inv accumulators [n], or null
@@ -113,6 +119,17 @@ __device__ __forceinline__ cx<T> adj_w(const FieldArgs<T>& a, int x, int y, int 
   return rmul(z < a.hi ? a.m1 : a.m3, eb);
 }
 
+// The images at x = 0 and y = 0 of the new H of cell (x, y, z).
+template <typename T> __device__ __forceinline__ void adj_images(const AdjArgs<T>& A, int x, int y, int z, const cx<T> h[3]) {
+  const FieldArgs<T>& a = A.f;
+  const Geo& g = a.g;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    if (x == g.nx) st<T>(A.ho + k * g.comp + g.at(0, y, z), cmul(a.pxm, h[k]));
+    if (y == g.ny) st<T>(A.ho + k * g.comp + g.at(x, 0, z), cmul(a.pym, h[k]));
+  }
+}
+
 // Adjoint of the H pass (plus the E pass transform deferred from the step
 // after it): Ebar += curl_b(V); the gradient term of the design cells.
 // Planes z0 .. z1 of the launch; UPML = false: neither they nor the planes
@@ -122,8 +139,12 @@ template <typename T, bool CURL, bool UPML> __global__ void __launch_bounds__(25
   const Geo& g = a.g;
   const int x = blockIdx.x * blockDim.x + threadIdx.x + 1;
   const int y = blockIdx.y * blockDim.y + threadIdx.y + 1;
-  const int z = A.z0 + blockIdx.z * blockDim.z + threadIdx.z;
-  if (x > g.nx || y > g.ny || z > A.z1) return;
+  int z = A.z0 + blockIdx.z * blockDim.z + threadIdx.z;
+  if (z > A.z1) {
+    z += A.z2 - A.z1 - 1;
+    if (z > A.z3) return;
+  }
+  if (x > g.nx || y > g.ny) return;
   const long i = g.at(x, y, z);
   cx<T> e[3];
 #pragma unroll
@@ -168,7 +189,7 @@ template <typename T, bool CURL, bool UPML> __global__ void __launch_bounds__(25
     }
   }
 #pragma unroll
-  for (int k = 0; k < 3; ++k) st<T>(a.e + k * g.comp + i, e[k]);
+  for (int k = 0; k < 3; ++k) st<T>(A.eo + k * g.comp + i, e[k]);
 }
 
 // Adjoint of the E pass (plus the H pass transform of the same step):
@@ -179,8 +200,12 @@ template <typename T, bool UPML> __global__ void __launch_bounds__(256) k_adj_e(
   const Geo& g = a.g;
   const int x = blockIdx.x * blockDim.x + threadIdx.x + 1;
   const int y = blockIdx.y * blockDim.y + threadIdx.y + 1;
-  const int z = A.z0 + blockIdx.z * blockDim.z + threadIdx.z;
-  if (x > g.nx || y > g.ny || z > A.z1) return;
+  int z = A.z0 + blockIdx.z * blockDim.z + threadIdx.z;
+  if (z > A.z1) {
+    z += A.z2 - A.z1 - 1;
+    if (z > A.z3) return;
+  }
+  if (x > g.nx || y > g.ny) return;
   const long i = g.at(x, y, z);
   cx<T> h[3];
 #pragma unroll
@@ -212,7 +237,40 @@ template <typename T, bool UPML> __global__ void __launch_bounds__(256) k_adj_e(
   h[1] = cadd(h[1], cadd(csub(csub(w0z, w[0]), w2x), w[2]));
   h[2] = cadd(h[2], cadd(csub(csub(w1x, w[1]), w0y), w[0]));
 #pragma unroll
-  for (int k = 0; k < 3; ++k) st<T>(a.h + k * g.comp + i, h[k]);
+  for (int k = 0; k < 3; ++k) st<T>(A.ho + k * g.comp + i, h[k]);
+  if (A.images) adj_images<T>(A, x, y, z, h);
+}
+
+// H's images of every plane, from the interior (ho = f.h).
+template <typename T> __global__ void __launch_bounds__(256) k_adj_images(AdjArgs<T> A) {
+  const Geo& g = A.f.g;
+  const int x = blockIdx.x * blockDim.x + threadIdx.x + 1;
+  const int y = blockIdx.y * blockDim.y + threadIdx.y + 1;
+  const int z = blockIdx.z * blockDim.z + threadIdx.z + 1;
+  if (x > g.nx || y > g.ny || z > g.nz || (x < g.nx && y < g.ny)) return;
+  cx<T> h[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) h[k] = ld<T>(A.f.h + k * g.comp + g.at(x, y, z));
+  adj_images<T>(A, x, y, z, h);
+}
+
+// The planes outside the slabs in one pass (FP32): E, H read and written once, 96
+// bytes a cell instead of 144.  160x160x352 on GB300: 148 us for 325 planes,
+// the two passes 201; with the slabs and the source 240 us a step, before 314.
+template <typename TL>
+__global__ void __launch_bounds__(MR_T, 2) k_adj_march(MarchArgs A, const __grid_constant__ MarchGrad J, int za, int zb,
+                                                       int zc) {
+  extern __shared__ __align__(128) unsigned char mr_dyn[];
+  const int z0 = za + zc * (int)blockIdx.z, z1 = min(z0 + zc - 1, zb);
+  march_tile<TL, false, true>(A, mr_dyn, blockIdx.x, blockIdx.y, z0, z1, nullptr, &J);
+}
+using AdjMarchFn = void (*)(MarchArgs, const MarchGrad, int, int, int);
+AdjMarchFn adj_march_kernel(int id) {
+#define IRIS_MARCH_K(ID, W, R) \
+  if (id == ID) return (AdjMarchFn)k_adj_march<MarchTile<W, R>>;
+  IRIS_MARCH_SHAPES(IRIS_MARCH_K)
+#undef IRIS_MARCH_K
+  return nullptr;
 }
 
 // Forward curl_b H of the E pass at the design cells (the H the next E pass
@@ -402,12 +460,13 @@ __global__ void __launch_bounds__(128) k_adj_sums(double2* __restrict__ src, con
   }
 }
 
-// One step's sums onto the adjoint fields.
+// One step's sums onto the adjoint fields, H's images included.
 __global__ void __launch_bounds__(128) k_adj_add(float2* __restrict__ ae, float2* __restrict__ ah, Geo g, AdjFace f,
-                                                 const double2* __restrict__ src) {
+                                                 const double2* __restrict__ src, cx<float> pxm, cx<float> pym) {
   const long L = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (L >= f.n) return;
-  const long i = g.at(f.x0 + (int)(L % f.nu), f.y0 + (int)(L / f.nu), f.z);
+  const int x = f.x0 + (int)(L % f.nu), y = f.y0 + (int)(L / f.nu);
+  const long i = g.at(x, y, f.z);
   float2* const dst[4] = {ae + i, ae + g.comp + i, ah + i, ah + g.comp + i};
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
@@ -416,6 +475,8 @@ __global__ void __launch_bounds__(128) k_adj_add(float2* __restrict__ ae, float2
     o.x = (float)(q == 1 || q == 2 ? (double)o.x - v.x : (double)o.x + v.x);
     o.y = (float)(q == 1 || q == 2 ? (double)o.y - v.y : (double)o.y + v.y);
     *dst[q] = o;
+    if (q >= 2 && x == g.nx) st<float>(dst[q] - g.nx, cmul(pxm, cx<float>{o.x, o.y}));
+    if (q >= 2 && y == g.ny) st<float>(dst[q] - g.ny * g.pitch, cmul(pym, cx<float>{o.x, o.y}));
   }
 }
 
@@ -451,6 +512,10 @@ struct iris_adjoint {
   int kmax[2] = {0, 0};                  // the largest weight's exponent
   bool src_scaled = false;               // d_ssx holds the forward pass's
   int src_cap = 1, src_it = 0, src_n = 0;
+  // FP32: the step's march, its slab kernels on st2 beside it
+  bool marched = false;
+  cudaStream_t st2 = nullptr;
+  cudaEvent_t fork = nullptr, join = nullptr;
   std::vector<void*> ckpt;     // per segment: e, h, d0, d1, b0, b1
   size_t fbytes = 0, sbytes[2] = {0, 0};
   int nsteps = 0;
@@ -475,6 +540,10 @@ template <typename T> AdjArgs<T> adj_args(const iris_adjoint* J, bool first, int
   A.f.pyp = conj(f.pym);
   A.f.pzp = conj(f.pzm);
   A.d = J->d;
+  A.eo = A.f.e;
+  A.ho = A.f.h;
+  A.z2 = 0;
+  A.z3 = -1;
   A.first = first ? 1 : 0;
   if (grad) {
     A.grad = J->d_grad;
@@ -501,6 +570,7 @@ template <typename T> void adj_source(iris_adjoint* J, int it) {
     J->src_it = it;
     J->src_n = std::min(J->src_cap, (it - std::max(p.to_fourier, 1)) / sf + 1);
   }
+  const AdjArgs<float> ph = adj_args<float>(J, false, -1, false);
   for (int side = 0; side < 2; ++side) {
     if (!J->side_on[side]) continue;
     AdjFace f{};
@@ -527,14 +597,60 @@ template <typename T> void adj_source(iris_adjoint* J, int it) {
           J->kmax[side]);
     }
     k_adj_add<<<nb, 128, 0, F->st>>>((float2*)J->A->e, (float2*)J->A->h, F->g, f,
-                                     J->d_src[side] + (long)((J->src_it - it) / sf) * 4 * f.n);
+                                     J->d_src[side] + (long)((J->src_it - it) / sf) * 4 * f.n, ph.f.pxm, ph.f.pym);
   }
   if (refill) J->src_scaled = true;
+}
+
+// Back to stepping in place.
+void adj_drop_march(iris_adjoint* J) {
+  cudaStreamSynchronize(J->F->st);
+  cudaGetLastError();
+  J->marched = false;
+  if (J->A->e2) cudaFree(J->A->e2);
+  if (J->A->h2) cudaFree(J->A->h2);
+  J->A->e2 = J->A->h2 = nullptr;
 }
 
 // Launch shape of planes z0 .. z1 (none when z1 < z0).
 dim3 adj_grid(const iris_engine* F, int z0, int z1) {
   return dim3(F->grd.x, F->grd.y, z1 < z0 ? 0u : (unsigned)((z1 - z0 + F->blk.z) / F->blk.z));
+}
+
+// One step with the planes pmlzi+2 .. pmlzf-2 marched: K1 of the planes below
+// and above (on the forward engine's second stream) beside them, then K2 of
+// the same planes, which reads W of both.
+void adj_step_march(iris_adjoint* J, bool first, int slot) {
+  iris_engine *F = J->F, *S = J->A;
+  const iris_params& p = F->p;
+  AdjArgs<float> a = adj_args<float>(J, first, slot, slot >= 0);
+  a.eo = (float2*)S->e2;
+  a.ho = (float2*)S->h2;
+  a.z0 = 1;
+  a.z1 = p.pmlzi + 1;
+  a.z2 = p.pmlzf - 1;
+  a.z3 = p.nz;
+  a.images = 1;
+  const int planes = a.z1 + a.z3 - a.z2 + 1;
+  const dim3 gr(F->grd.x, F->grd.y, (unsigned)((planes + F->blk.z - 1) / F->blk.z));
+  MarchArgs m{};
+  m.f = a.f;
+  m.e_new = a.eo;
+  m.h_new = a.ho;
+  m.tx = S->mshape.tx;
+  m.ty = S->mshape.ty;
+  const MarchGrad G{a.d.x0, a.d.y0, a.d.z0, a.d.nx, a.d.ny, a.d.nz, a.d.n, a.rec, a.grad};
+  const int za = p.pmlzi + 2, zb = p.pmlzf - 2, zc = march_chunk(zb - za + 1);
+  cudaEventRecord(J->fork, F->st);
+  cudaStreamWaitEvent(J->st2, J->fork, 0);
+  k_adj_h<float, true, true><<<gr, F->blk, 0, J->st2>>>(a);
+  adj_march_kernel(S->mshape.id)<<<dim3(m.tx, m.ty, (zb - za + zc) / zc), MR_T, S->mshape.smem, F->st>>>(m, G, za, zb, zc);
+  cudaEventRecord(J->join, J->st2);
+  cudaStreamWaitEvent(F->st, J->join, 0);
+  a.f.e = a.eo;  // K2 reads the new E
+  k_adj_e<float, true><<<gr, F->blk, 0, F->st>>>(a);
+  std::swap(S->e, S->e2);
+  std::swap(S->h, S->h2);
 }
 
 // One adjoint step (K1 then K2) for forward step it; rec slot or -1.  Each
@@ -544,6 +660,7 @@ template <typename T> void adj_step(iris_adjoint* J, bool first, int slot) {
   iris_engine* F = J->F;
   const iris_params& p = F->p;
   const bool grad = slot >= 0;
+  if (J->marched) return adj_step_march(J, first, slot);
   AdjArgs<T> a = adj_args<T>(J, first, slot, grad);
   auto k1 = [&](int z0, int z1, bool upml) {
     a.z0 = z0;
@@ -606,13 +723,40 @@ int zero_state(iris_engine* E, size_t fbytes, const size_t* sbytes) {
   return IRIS_OK;
 }
 
+// Second buffers and launch of the march, where its offsets reach, there are
+// planes to march and memory allows.
+void adj_setup_march(iris_adjoint* J) {
+  iris_engine* S = J->A;
+  const iris_params& p = J->F->p;
+  if (J->F->prec != IRIS_FP32 || 3 * S->g.comp >= (1L << 31) || p.pmlzf - 2 < p.pmlzi + 2) return;
+  S->mshape = march_shape(p.nx, p.ny);
+  int lo = 0, hi = 0;
+  cudaDeviceGetStreamPriorityRange(&lo, &hi);
+  J->marched = cudaMalloc(&S->e2, J->fbytes) == cudaSuccess && cudaMalloc(&S->h2, J->fbytes) == cudaSuccess &&
+               cudaMemsetAsync(S->e2, 0, J->fbytes, J->F->st) == cudaSuccess &&
+               cudaMemsetAsync(S->h2, 0, J->fbytes, J->F->st) == cudaSuccess &&
+               cudaStreamCreateWithPriority(&J->st2, cudaStreamNonBlocking, hi) == cudaSuccess &&
+               cudaEventCreateWithFlags(&J->fork, cudaEventDisableTiming) == cudaSuccess &&
+               cudaEventCreateWithFlags(&J->join, cudaEventDisableTiming) == cudaSuccess &&
+               cudaFuncSetAttribute((const void*)adj_march_kernel(S->mshape.id),
+                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S->mshape.smem) == cudaSuccess;
+  if (!J->marched) adj_drop_march(J);
+}
+
 template <typename T> int adj_forward(iris_adjoint* J, int nsteps) {
   iris_engine* F = J->F;
   const int S = (nsteps + J->K - 1) / J->K;
   const size_t cbytes = 2 * J->fbytes + 2 * (J->sbytes[0] + J->sbytes[1]);
   while ((int)J->ckpt.size() < S) {
     void* q = nullptr;
-    if (cudaMalloc(&q, cbytes) != cudaSuccess) {
+    cudaError_t e = cudaMalloc(&q, cbytes);
+    if (e != cudaSuccess && J->marched) {
+      // the checkpoints come first: step in place, without the second buffers
+      cudaGetLastError();
+      adj_drop_march(J);
+      e = cudaMalloc(&q, cbytes);
+    }
+    if (e != cudaSuccess) {
       cudaGetLastError();
       return fail(IRIS_ENOMEM, "checkpoint allocation failed (" + std::to_string(S) + " checkpoints of " +
                                    std::to_string(cbytes) + " bytes)");
@@ -702,8 +846,9 @@ void adj_free(iris_adjoint* J) {
     if (q) cudaFree(q);
   for (void* q : J->ckpt)
     if (q) cudaFree(q);
-  for (cudaEvent_t e : J->ev)
+  for (cudaEvent_t e : {J->ev[0], J->ev[1], J->fork, J->join})
     if (e) cudaEventDestroy(e);
+  if (J->st2) cudaStreamDestroy(J->st2);
 }
 
 }  // namespace
@@ -812,6 +957,7 @@ int iris_adjoint_create(const iris_params* pin, const double* fw, const int desi
   if (cudaMemcpy(J->d_w, wd.data(), sizeof(double) * 2 * nof, cudaMemcpyHostToDevice) != cudaSuccess ||
       cudaEventCreate(&J->ev[0]) != cudaSuccess || cudaEventCreate(&J->ev[1]) != cudaSuccess)
     return bail(fail(IRIS_ECUDA, "adjoint initialisation failed"));
+  adj_setup_march(J);
   *out = J;
   return IRIS_OK;
 }
@@ -902,6 +1048,10 @@ int iris_adjoint_apply(iris_adjoint* J, int nsteps) {
   CK(cudaSetDevice(F->device));
   CK(cudaStreamSynchronize(J->A->st));
   const bool d = F->prec == IRIS_FP64;
+  if (J->marched && nsteps > 0) {  // the caller's state may hold any images
+    const AdjArgs<float> a = adj_args<float>(J, false, -1, false);
+    k_adj_images<float><<<F->grd, F->blk, 0, F->st>>>(a);
+  }
   for (int k = 0; k < nsteps; ++k) d ? adj_step<double>(J, k == 0, -1) : adj_step<float>(J, k == 0, -1);
   if (nsteps > 0) d ? adj_finalize<double>(J) : adj_finalize<float>(J);
   CK(cudaGetLastError());

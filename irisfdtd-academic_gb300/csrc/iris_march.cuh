@@ -61,6 +61,17 @@ struct MarchSlabArgs {
   float2* d_new[2];
 };
 
+// The adjoint's march (ADJ): the same column with the passes' roles exchanged,
+// E' = E - dtcq2 curl_b H, then H' = H + curl_f W, W = m E' (m the structure's
+// eps_inv, 1/eps1 or 1/eps3); W takes E's place in the ring.  E has no stored
+// images.  The gradient term of the design cells, with the forward curl rec.
+struct MarchGrad {
+  int x0, y0, z0, nx, ny, nz;  // design cells
+  long n;
+  const float2* rec;  // [3][n]
+  double* grad;       // [n], or null
+};
+
 __device__ __forceinline__ void march_cpa16(unsigned dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
@@ -85,9 +96,9 @@ template <int W_, int R_, int T_ = MR_T, bool UPML_ = false> struct MarchTile {
 
 // Planes z0..z1 of tile (bx, by): every thread of the CTA.  EDGE: the tile
 // touches a border of the plane.
-template <typename TL, bool CEPS, bool EDGE>
+template <typename TL, bool CEPS, bool EDGE, bool ADJ>
 __device__ __forceinline__ void march_column(const MarchArgs& A, unsigned char* smem, int bx, int by, int z0, int z1,
-                                             float2* const* d_new = nullptr) {
+                                             float2* const* d_new, const MarchGrad* J) {
   const FieldArgs<float>& a = A.f;
   const Geo& g = a.g;
   constexpr int HC = TL::HC, EC = TL::EC, BXH = TL::BXH, BXE = TL::BXE, NI = TL::NI;
@@ -309,6 +320,9 @@ __device__ __forceinline__ void march_column(const MarchArgs& A, unsigned char* 
         const cx<float> dv[3] = {get(u + t), get(u + TL::T + t), get(u + 2 * TL::T + t)};
         e_apply<float, CEPS, 7, !CEPS, true>(a, own[s] && z <= z1 ? d_new : nullptr, px, py, zc, cu, en, 0.f, dv,
                                              (const float*)(u + 6 * TL::T));
+      } else if (ADJ) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) en[k] = cadd(en[k], rmul(-a.dtcq2, cu[k]));
       } else if (CEPS && mat) {
 #pragma unroll
         for (int k = 0; k < 3; ++k) en[k] = cadd(en[k], cmul(epc[CEPS ? s : 0], cu[k]));
@@ -327,6 +341,27 @@ __device__ __forceinline__ void march_column(const MarchArgs& A, unsigned char* 
       if (UPML && z == g.nz + 1) {
 #pragma unroll
         for (int k = 0; k < 3; ++k) en[k] = cmul(a.pzp, en[k]);
+      }
+      if (ADJ) {
+        if (own[s] && z <= z1) {
+          const int i = z * pl + ow[s];
+#pragma unroll
+          for (int k = 0; k < 3; ++k) st<float>(A.e_new + (k * cp + i), en[k]);
+          const int c = t + s * TL::T, dx = x0 + c % TL::WT - J->x0, dy = y0 + c / TL::WT - J->y0, dz = z - J->z0;
+          if (J->grad && dz >= 0 && dz < J->nz && dx >= 0 && dx < J->nx && dy >= 0 && dy < J->ny) {
+            const long q = ((long)dz * J->ny + dy) * J->nx + dx;
+            float g1 = 0.f;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+              const cx<float> r = get(J->rec + k * J->n + q);
+              g1 = add_(g1, add_(mul_(en[k].re, r.re), mul_(en[k].im, r.im)));
+            }
+            J->grad[q] += (double)g1;
+          }
+        }
+        const float m = mat ? ep[s] : mz;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) en[k] = rmul(m, en[k]);  // W from here on
       }
 #pragma unroll
       for (int k = 0; k < 3; ++k) ez[ie[s] + k * EC] = make_float2(en[k].re, en[k].im);
@@ -351,6 +386,10 @@ __device__ __forceinline__ void march_column(const MarchArgs& A, unsigned char* 
             const float2* u = (const float2*)(su + (z & 3) * TL::UB);
             const cx<float> bv[3] = {get(u + 3 * TL::T + t), get(u + 4 * TL::T + t), get(u + 5 * TL::T + t)};
             h_update<float, true>(a, px, py, z - 1, ev[s], xp, yp, zp, hn, bv, (const float*)(u + 6 * TL::T) + NCOEF);
+          } else if (ADJ) {
+            hn[0] = cadd(hn[0], cadd(csub(csub(yp[2], ev[s][2]), zp[1]), ev[s][1]));
+            hn[1] = cadd(hn[1], cadd(csub(csub(zp[0], ev[s][0]), xp[2]), ev[s][2]));
+            hn[2] = cadd(hn[2], cadd(csub(csub(xp[1], ev[s][1]), yp[0]), ev[s][0]));
           } else {
             h_update<float, false>(a, 1, 1, 1, ev[s], xp, yp, zp, hn);
           }
@@ -367,19 +406,19 @@ __device__ __forceinline__ void march_column(const MarchArgs& A, unsigned char* 
           if (EDGE && (ed[s] & 1)) {
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
-              st<float>(A.e_new + (k * cp + j - g.nx), cmul(a.pxm, ev[s][k]));
+              if (!ADJ) st<float>(A.e_new + (k * cp + j - g.nx), cmul(a.pxm, ev[s][k]));
               st<float>(A.h_new + (k * cp + j - g.nx), cmul(a.pxm, hn[k]));
             }
           }
           if (EDGE && (ed[s] & 2)) {
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
-              st<float>(A.e_new + (k * cp + j - g.ny * pt), cmul(a.pym, ev[s][k]));
+              if (!ADJ) st<float>(A.e_new + (k * cp + j - g.ny * pt), cmul(a.pym, ev[s][k]));
               st<float>(A.h_new + (k * cp + j - g.ny * pt), cmul(a.pym, hn[k]));
             }
           }
         }
-        if (z <= z1) {
+        if (!ADJ && z <= z1) {
 #pragma unroll
           for (int k = 0; k < 3; ++k) st<float>(A.e_new + (k * cp + i), en[k]);
           if (UPML && z == 1) {
@@ -409,13 +448,13 @@ __device__ __forceinline__ void march_column(const MarchArgs& A, unsigned char* 
   __syncthreads();
 }
 
-template <typename TL, bool CEPS>
+template <typename TL, bool CEPS, bool ADJ = false>
 __device__ __forceinline__ void march_tile(const MarchArgs& A, unsigned char* smem, int bx, int by, int z0, int z1,
-                                           float2* const* d_new = nullptr) {
+                                           float2* const* d_new = nullptr, const MarchGrad* J = nullptr) {
   if (bx == 0 || by == 0 || bx == A.tx - 1 || by == A.ty - 1)
-    march_column<TL, CEPS, true>(A, smem, bx, by, z0, z1, d_new);
+    march_column<TL, CEPS, true, ADJ>(A, smem, bx, by, z0, z1, d_new, J);
   else
-    march_column<TL, CEPS, false>(A, smem, bx, by, z0, z1, d_new);
+    march_column<TL, CEPS, false, ADJ>(A, smem, bx, by, z0, z1, d_new, J);
 }
 
 // The tile shapes, and the one taken for an nx x ny plane: the fewest bytes of
