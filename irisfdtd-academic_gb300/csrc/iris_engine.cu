@@ -2457,6 +2457,8 @@ template <typename T> int step_t(iris_engine* E, int it0, int n) {
 
 // The kernel of a resident engine.
 template <typename T> const void* res_kernel(const iris_engine* E, bool cplx) {
+  if constexpr (std::is_same<T, double>::value)
+    if (E->res_ll) return cplx ? (const void*)k_res<double, true, 6, true> : (const void*)k_res<double, false, 6, true>;
   if (E->res_nc == 6) return cplx ? (const void*)k_res<T, true, 6> : (const void*)k_res<T, false, 6>;
   return cplx ? (const void*)k_res<T, true, 5> : (const void*)k_res<T, false, 5>;
 }
@@ -2562,6 +2564,7 @@ int res_setup(iris_engine* E) {
     E->res_head = (int)head;
     E->res_smem = head + most;
     E->res_threads = (int)std::min<size_t>(RES_THREADS, std::max<size_t>(64, (items + 31) / 32 * 32));
+    E->res_ll = E->prec == IRIS_FP64 && nc == 6 && items <= (size_t)RES_LL_THREADS;
     fits = true;
   }
   if (!fits) return IRIS_OK;
@@ -2576,16 +2579,21 @@ int res_setup(iris_engine* E) {
   }
   CK(cudaMalloc(&E->d_rcta, sizeof(ResCta) * G));
   CK(cudaMalloc(&E->d_rflag, sizeof(unsigned) * RES_FLAG_STRIDE * G));
+  if (E->res_ll) {
+    const size_t b = sizeof(ulonglong2) * 12 * (size_t)E->g.comp;
+    CK(cudaMalloc(&E->d_rll, b));
+    CK(cudaMemsetAsync(E->d_rll, 0, b, E->st));
+  }
   E->res = true;
   return IRIS_OK;
 }
 
 // Microseconds of an FP64 step, as measured on GB300: the resident kernel by
 // its busiest CTA, 18 ns a cell and twice that in the UPML (256x4x340, 2290
-// cells a CTA, 47 us; 2600x1x16, a UPML row of 2600 on a CTA, 95); k_tiny 0.24
-// ns a cell and its barriers (20x20x1000 93, 128x128x60 194); the split passes
-// 0.15 to 0.2 ns a cell and the launches (2600x1x16 36, 20x20x1000 71,
-// 70x70x70 70, 128x128x60 160).
+// cells a CTA, 47 us; 2600x1x16, a UPML row of 2600 on a CTA, 95); k_tiny 0.19
+// ns a cell and its barriers (2600x1x16 27, 2600x1x64 53, 20x20x1000 93); the
+// split passes 0.15 ns a cell and the launches (2600x1x16 32, 2600x1x64 45,
+// 70x70x70 67, 20x20x1000 67).
 double res_us64(const iris_engine* E) {
   const iris_params& p = E->p;
   long most = 0;
@@ -2596,9 +2604,9 @@ double res_us64(const iris_engine* E) {
   }
   return 5.0 + 0.018 * most;
 }
-double tiny_us64(const iris_engine* E) { return 5.0 + 2.4e-4 * E->p.nx * E->p.ny * E->p.nz; }
+double tiny_us64(const iris_engine* E) { return 16.0 + 1.93e-4 * E->p.nx * E->p.ny * E->p.nz; }
 double split_us64(const iris_engine* E) {
-  return std::max(36.0, 10.0 + 1.8e-4 * E->p.nx * E->p.ny * E->p.nz);
+  return std::max(32.0, 14.0 + 1.5e-4 * E->p.nx * E->p.ny * E->p.nz);
 }
 
 // The sample points of every CTA, E then H, each in ring order: shared-memory
@@ -2734,6 +2742,9 @@ template <typename T> int step_persist(iris_engine* E, int it0, int n) {
           B.one[k] = E->ph[k][0] == 1.0 && E->ph[k][1] == 0.0 && E->ph[3 + k][0] == 1.0 && E->ph[3 + k][1] == 0.0;
         B.flag = E->d_rflag;
         B.err = E->d_err;
+        B.ll = E->d_rll;
+        B.ep = E->res_ep;
+        E->res_ep += span;
         long long limit = STREAM_WAIT_CYCLES;
         void* rargs[] = {&B, &limit};
         CK(cudaMemsetAsync(E->d_rflag, 0, sizeof(unsigned) * RES_FLAG_STRIDE * E->res_blocks, E->st));
@@ -3164,7 +3175,7 @@ void free_engine(iris_engine* E) {
   void* ptrs[] = {E->e, E->h, E->pml_d[0], E->pml_d[1], E->pml_b[0], E->pml_b[1], E->coef, E->eps, E->d_segs,
                   E->S, E->d_tk, E->d_fw, E->fd, E->d_wt, E->d_faces, E->d_J, E->e2, E->h2, E->pml_d2[0],
                   E->pml_d2[1], E->d_err, E->d_it, E->d_wtc, E->d_wt64, E->d_part, E->d_bar, E->d_stage,
-                  E->d_tfv, E->d_sidx, E->d_rcta, E->d_rsamp, E->d_rflag};
+                  E->d_tfv, E->d_sidx, E->d_rcta, E->d_rsamp, E->d_rflag, E->d_rll};
   for (void* q : ptrs)
     if (q) cudaFree(q);
   if (E->h_J) cudaFreeHost(E->h_J);

@@ -129,7 +129,7 @@ struct iris_engine {
   long* d_sidx = nullptr;  // its DFT sample points: storage index * 8 + field
   // the resident form of it (k_res): grids whose E and H fit in shared memory
   bool res = false;
-  bool res_runs = false;
+  bool res_runs = false, res_ll = false;
   int res_nc = 6, res_db = 1, res_rows = 0, res_nruns = 0, res_head = 0, res_blocks = 0, res_threads = 0;
   size_t res_smem = 0;
   iris::ResSrc res_src{};
@@ -137,6 +137,8 @@ struct iris_engine {
   iris::ResCta* d_rcta = nullptr;
   uint2* d_rsamp = nullptr;
   unsigned* d_rflag = nullptr;
+  ulonglong2* d_rll = nullptr;    // its packets (null: not the LL form) and the tags given out
+  unsigned long long res_ep = 0;
   // staging buffer of the complex(8) field transfers (allocated on first use)
   void* d_stage = nullptr;
   size_t stage_bytes = 0;
