@@ -84,6 +84,16 @@ template <typename T> struct cx { T re, im; };
 
 __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 
+// Programmatic launch order: the grids before this one in its stream are done
+// (a no-op in a plain launch); then the next may start its CTAs as this one's
+// last ones run, to wait here in turn.  Every thread of a kernel that is
+// launched this way calls it before it touches memory, so a grid past it has
+// all earlier ones behind it.
+__device__ __forceinline__ void grid_order() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // mbarriers (shared memory, this CTA) and their bounded wait.
 __device__ __forceinline__ void mbar_init(uint64_t* bar, unsigned count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
