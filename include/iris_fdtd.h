@@ -169,18 +169,17 @@ typedef struct iris_params {
  * TF/SF, DFT sample), the state in shared memory where it fits, the passes
  * separated by flags between neighbours or by grid-wide barriers; the split
  * passes' arithmetic, so the same results bit for bit.  The default for
- * IRIS_FP64 grids of at most IRIS_PERSISTENT_MAX_CELLS cells that it is
- * estimated to step faster than the split passes (in effect those that fit in
- * shared memory, up to about 350 thousand cells) and for IRIS_FP32 grids of at
- * most IRIS_PERSISTENT_MAX_CELLS_FP32 cells (up to those sizes it steps at
- * least as fast as the split and the fused passes: at 160x160x200, 5.1 million
- * cells, 161, 160 and 158 us a step, at 256x256x128 262, 244 and 236, at
- * 160x160x100 89, 93 and 92); asked for explicitly, grids of fewer than
- * 2^31 / 3 cells on a device with cooperative launches (else iris_create
- * returns IRIS_EINVAL)                                                    */
+ * grids of at most IRIS_PERSISTENT_MAX_CELLS cells in IRIS_FP64, or
+ * IRIS_PERSISTENT_MAX_CELLS_FP32 in IRIS_FP32, that it is estimated to step
+ * faster than the split passes (in effect those that fit in shared memory, up
+ * to about 350 thousand cells in IRIS_FP64 and 800 thousand in IRIS_FP32);
+ * above, IRIS_FP64 takes the split passes, IRIS_FP32 the split passes up to
+ * 2.25 x 2^20 cells (and on thin grids) and the fused pass beyond.  Asked for
+ * explicitly, grids of fewer than 2^31 / 3 cells on a device with cooperative
+ * launches (else iris_create returns IRIS_EINVAL)                         */
 #define IRIS_STENCIL_PERSISTENT 4
 #define IRIS_PERSISTENT_MAX_CELLS 1048576
-#define IRIS_PERSISTENT_MAX_CELLS_FP32 5242880
+#define IRIS_PERSISTENT_MAX_CELLS_FP32 1048576
 
 typedef struct iris_engine iris_engine;
 

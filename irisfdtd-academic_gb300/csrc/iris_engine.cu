@@ -71,6 +71,7 @@ __global__ void __launch_bounds__(256) k_update_h64(FieldArgs<double> a) {
 
 // The FP32 split passes.
 template <bool CEPS> __global__ void __launch_bounds__(256) k_update_e(FieldArgs<float> a) {
+  grid_order();
   const int x = blockIdx.x * blockDim.x + threadIdx.x + 1;
   const int y = blockIdx.y * blockDim.y + threadIdx.y + 1;
   const int z = blockIdx.z * blockDim.z + threadIdx.z + 1;
@@ -79,6 +80,7 @@ template <bool CEPS> __global__ void __launch_bounds__(256) k_update_e(FieldArgs
 }
 
 __global__ void __launch_bounds__(256) k_update_h(FieldArgs<float> a) {
+  grid_order();
   const int x = blockIdx.x * blockDim.x + threadIdx.x + 1;
   const int y = blockIdx.y * blockDim.y + threadIdx.y + 1;
   const int z = blockIdx.z * blockDim.z + threadIdx.z + 1;
@@ -2033,6 +2035,7 @@ __global__ void __launch_bounds__(FZ_X* FZ_Y, 2) k_fused(FusedArgs A) {
 // blockIdx.z covers zc planes.
 template <typename TL, bool CEPS> __global__ void __launch_bounds__(MR_T, 2) k_march(MarchArgs A, int za, int zb, int zc) {
   extern __shared__ __align__(128) unsigned char mr_dyn[];
+  grid_order();
   const int z0 = za + zc * (int)blockIdx.z, z1 = min(z0 + zc - 1, zb);
   march_tile<TL, CEPS>(A, mr_dyn, blockIdx.x, blockIdx.y, z0, z1);
 }
@@ -2211,17 +2214,23 @@ int validate(const iris_params& p) {
 // CTAs are set up while the grid before it drains.  Three to four launches a
 // step lose 2 us each without: 256x4x768 in FP64 115 us a step, 106 so.
 template <typename... P, typename... A>
-void launch_ordered(void (*k)(P...), dim3 grid, dim3 block, cudaStream_t st, A... args) {
+void launch_ordered_smem(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
   cudaLaunchAttribute at{};
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t c{};
   c.gridDim = grid;
   c.blockDim = block;
+  c.dynamicSmemBytes = smem;
   c.stream = st;
   c.attrs = &at;
   c.numAttrs = 1;
   cudaLaunchKernelEx(&c, k, P(args)...);
+}
+
+template <typename... P, typename... A>
+void launch_ordered(void (*k)(P...), dim3 grid, dim3 block, cudaStream_t st, A... args) {
+  launch_ordered_smem(k, grid, block, 0, st, args...);
 }
 
 // CTAs of the FP64 split passes (memory keeps the cells below 2^32 - 256).
@@ -2235,8 +2244,7 @@ template <typename T> void launch_e(iris_engine* E) {
       k_stream_e<<<E->sgrd, dim3(SX, SY), STREAM_SMEM_E, E->st>>>(a, E->d_err);
       return;
     }
-    if (E->eps_complex) k_update_e<true><<<E->grd, E->blk, 0, E->st>>>(a);
-    else k_update_e<false><<<E->grd, E->blk, 0, E->st>>>(a);
+    launch_ordered(E->eps_complex ? k_update_e<true> : k_update_e<false>, E->grd, E->blk, E->st, a);
   } else {
     launch_ordered(E->eps_complex ? k_update_e64<true> : k_update_e64<false>, blocks64(E), 256, E->st, a);
   }
@@ -2249,7 +2257,7 @@ template <typename T> void launch_h(iris_engine* E) {
       return;
     }
   }
-  if constexpr (std::is_same<T, float>::value) k_update_h<<<E->grd, E->blk, 0, E->st>>>(field_args<float>(E));
+  if constexpr (std::is_same<T, float>::value) launch_ordered(k_update_h, E->grd, E->blk, E->st, field_args<float>(E));
   else launch_ordered(k_update_h64, blocks64(E), 256, E->st, field_args<double>(E));
 }
 // The TF/SF table of steps it .. it+n-1 (at most tfv_cap), from *itp on when
@@ -2350,6 +2358,12 @@ FusedArgs fused_args(const iris_engine* E, int part) {
   return a;
 }
 
+// Cells above which FP32 takes the fused pass: its shorter chain of launches and
+// 12 values a cell win over the L2-resident split passes from here (us a step,
+// fused and split: 128x128x110 60 and 57, 128x128x128 67.5 and 65.9, 300x20x400
+// 69 and 74, 160x160x100 74 and 80, 128x128x256 112 and 121; the persistent
+// kernel 63, 76, 78, 91 and 135).
+constexpr long FUSED_MIN_CELLS = 9L << 18;
 // Share of the fused pass's threads that own a cell of an nx x ny plane
 // (each 32 x 16 tile writes 31 x 15 cells).
 double fused_fill(int nx, int ny) {
@@ -2372,7 +2386,8 @@ void fused_chunks(std::vector<int>& r, int za, int zb, long tiles) {
 // The march of planes (za, zb, zc, n).
 void launch_march(iris_engine* E, const std::vector<int>& r, cudaStream_t st) {
   const MarchArgs a = march_args(E);
-  march_kernel(E->mshape.id, E->eps_complex)<<<dim3(a.tx, a.ty, r[3]), MR_T, E->mshape.smem, st>>>(a, r[0], r[1], r[2]);
+  launch_ordered_smem(march_kernel(E->mshape.id, E->eps_complex), dim3(a.tx, a.ty, r[3]), MR_T, E->mshape.smem, st, a, r[0],
+                      r[1], r[2]);
 }
 // The slabs' (one or two ranges).
 void launch_slabs(iris_engine* E, const std::vector<int>& r, cudaStream_t st) {
@@ -2613,22 +2628,29 @@ int res_setup(iris_engine* E) {
 // its busiest CTA, 18 ns a cell and twice that in the UPML (256x4x340, 2290
 // cells a CTA, 47 us; 2600x1x16, a UPML row of 2600 on a CTA, 95); k_tiny 0.19
 // ns a cell and its barriers (2600x1x16 27, 2600x1x64 53, 20x20x1000 93); the
-// split passes 0.15 ns a cell and the launches (2600x1x16 32, 2600x1x64 45,
-// 70x70x70 67, 20x20x1000 67).
-double res_us64(const iris_engine* E) {
+// split passes 0.14 ns a cell and the launches (2600x1x16 26, 2600x1x40 28,
+// 70x70x70 60, 20x20x1000 59).
+long res_busiest(const iris_engine* E, int row) {
   const iris_params& p = E->p;
   long most = 0;
   for (const ResCta& c : E->res_cta) {
     long n = 0;
     for (long r = c.r0; r < c.r1; ++r) n += r / p.ny < p.pmlzi || r / p.ny + 1 >= p.pmlzf ? 2 : 1;
-    most = std::max(most, n * p.nx);
+    most = std::max(most, n * row);
   }
-  return 5.0 + 0.018 * most;
+  return most;
 }
+double res_us64(const iris_engine* E) { return 5.0 + 0.018 * res_busiest(E, E->p.nx); }
 double tiny_us64(const iris_engine* E) { return 16.0 + 1.93e-4 * E->p.nx * E->p.ny * E->p.nz; }
 double split_us64(const iris_engine* E) {
-  return std::max(32.0, 14.0 + 1.5e-4 * E->p.nx * E->p.ny * E->p.nz);
+  return std::max(26.0, 11.0 + 1.4e-4 * E->p.nx * E->p.ny * E->p.nz);
 }
+
+// The same in FP32: 2.1 ns a lane of its 32-cell runs (2600x1x130 10.9 us,
+// 5000x1x40 20.4, 256x4x650 9.6), split passes 20 ps a cell and the launches
+// (2600x1x130 15.3, 5000x1x40 12.8, 256x4x650 16.5, 64x64x200 19.1; k_tiny 20.7).
+double res_us32(const iris_engine* E) { return 0.0021 * res_busiest(E, (E->p.nx + 31) / 32 * 32); }
+double split_us32(const iris_engine* E) { return 8.5 + 2e-5 * E->p.nx * E->p.ny * E->p.nz; }
 
 // The sample points of every CTA, E then H, each in ring order: shared-memory
 // offset (E_x outside it: storage index) with its flags, and ring position.
@@ -3318,13 +3340,13 @@ int create_engine(const iris_params* pin, const double* fw, bool member, bool z_
   E->grd = dim3((p.nx + bx - 1) / bx, (p.ny + by - 1) / by, (p.nz + bz - 1) / bz);
   E->src = make_src(p);
   // Small grids step with the persistent kernel (asked for, or by default
-  // when the device runs cooperative launches: FP64 grids of at most
-  // IRIS_PERSISTENT_MAX_CELLS cells that it is estimated to step faster,
-  // FP32 grids of at most IRIS_PERSISTENT_MAX_CELLS_FP32); otherwise FP32 steps with the fused E+H pass unless the split or
-  // streamed passes are asked for, or unless the fused pass's 32 x 16 tiles
-  // would leave more than half of their threads idle on the grid's x-y
-  // plane (rows or columns short of a tile: the split passes then); FP64
-  // steps with the split passes.
+  // when the device runs cooperative launches, the grid has at most
+  // IRIS_PERSISTENT_MAX_CELLS[_FP32] cells and it is estimated to step
+  // faster); otherwise FP64 steps with the split passes, and FP32 with the
+  // fused E+H pass unless the split or streamed passes are asked for, the grid
+  // is small, or the fused pass's 32 x 16 tiles would leave more than half of
+  // their threads idle on the grid's x-y plane (rows or columns short of a
+  // tile): the split passes then.
   {
     int coop = 0, nsm = 0, occ = 0;
     cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, E->device);
@@ -3370,10 +3392,14 @@ int create_engine(const iris_params* pin, const double* fw, bool member, bool z_
       const double res = E->res ? res_us64(E) : 1e300, tiny = tiny_us64(E);
       if (res > tiny) E->res = false;
       if (p.stencil == IRIS_STENCIL_DEFAULT && std::min(res, tiny) > split_us64(E)) E->persist = E->res = false;
+    } else if (p.stencil == IRIS_STENCIL_DEFAULT && !(E->res && res_us32(E) <= split_us32(E))) {
+      E->persist = E->res = false;
     }
   }
   E->fused = !E->persist && E->prec == IRIS_FP32 &&
-             (p.stencil == IRIS_STENCIL_FUSED || (p.stencil == IRIS_STENCIL_DEFAULT && fused_fill(p.nx, p.ny) >= 0.5));
+             (p.stencil == IRIS_STENCIL_FUSED ||
+              (p.stencil == IRIS_STENCIL_DEFAULT && (long)p.nx * p.ny * p.nz > FUSED_MIN_CELLS &&
+               fused_fill(p.nx, p.ny) >= 0.5));
   if (E->fused) {
     if (cudaMalloc(&E->e2, fbytes) != cudaSuccess || cudaMalloc(&E->h2, fbytes) != cudaSuccess)
       return bail(fail(IRIS_ENOMEM, "second field buffers: allocation failed"));
