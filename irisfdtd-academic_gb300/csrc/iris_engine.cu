@@ -2630,27 +2630,36 @@ int res_setup(iris_engine* E) {
 // ns a cell and its barriers (2600x1x16 27, 2600x1x64 53, 20x20x1000 93); the
 // split passes 0.14 ns a cell and the launches (2600x1x16 26, 2600x1x40 28,
 // 70x70x70 60, 20x20x1000 59).
-long res_busiest(const iris_engine* E, int row) {
+double res_busiest(const iris_engine* E, double upml) {  // cells, a UPML one weighing upml
   const iris_params& p = E->p;
-  long most = 0;
+  double most = 0;
   for (const ResCta& c : E->res_cta) {
-    long n = 0;
-    for (long r = c.r0; r < c.r1; ++r) n += r / p.ny < p.pmlzi || r / p.ny + 1 >= p.pmlzf ? 2 : 1;
-    most = std::max(most, n * row);
+    double n = 0;
+    for (long r = c.r0; r < c.r1; ++r) n += r / p.ny < p.pmlzi || r / p.ny + 1 >= p.pmlzf ? upml : 1.0;
+    most = std::max(most, n * p.nx);
   }
   return most;
 }
-double res_us64(const iris_engine* E) { return 5.0 + 0.018 * res_busiest(E, E->p.nx); }
+double res_us64(const iris_engine* E) { return 5.0 + 0.018 * res_busiest(E, 2.0); }
 double tiny_us64(const iris_engine* E) { return 16.0 + 1.93e-4 * E->p.nx * E->p.ny * E->p.nz; }
 double split_us64(const iris_engine* E) {
   return std::max(26.0, 11.0 + 1.4e-4 * E->p.nx * E->p.ny * E->p.nz);
 }
 
-// The same in FP32: 2.1 ns a lane of its 32-cell runs (2600x1x130 10.9 us,
-// 5000x1x40 20.4, 256x4x650 9.6), split passes 20 ps a cell and the launches
-// (2600x1x130 15.3, 5000x1x40 12.8, 256x4x650 16.5, 64x64x200 19.1; k_tiny 20.7).
-double res_us32(const iris_engine* E) { return 0.0021 * res_busiest(E, (E->p.nx + 31) / 32 * 32); }
-double split_us32(const iris_engine* E) { return 8.5 + 2e-5 * E->p.nx * E->p.ny * E->p.nz; }
+// The same in FP32, by lanes (rows rounded up to warps): the resident kernel
+// 1.35 ns a lane of its busiest CTA, 1.5 more where the row above and below is
+// another CTA's, a quarter more with E_x in global memory (64x8x1300 9.0,
+// 64x64x120 12.2, 2600x1x130 10.9, 5000x1x40 20.4, 61x82x154 24.5); the split
+// passes 13.5 ps a lane and the launches (15.8, 14.9, 15.3, 13.0, 19.6; k_tiny
+// is slower than they are: 64x64x200 20.7 against 19.1).
+double lanes32(const iris_engine* E) { return (double)((E->p.nx + 31) / 32 * 32) / E->p.nx; }
+double res_us32(const iris_engine* E) {
+  const double far = std::min(1.0, (double)E->res_blocks / E->p.nz);  // rows of a plane to rows of a CTA
+  return 1e-3 * lanes32(E) * res_busiest(E, 1.5) * (1.35 + 1.5 * far) * (E->res_nc == 5 ? 1.25 : 1.0);
+}
+double split_us32(const iris_engine* E) {
+  return 8.0 + 1.35e-5 * lanes32(E) * E->p.nx * E->p.ny * E->p.nz;
+}
 
 // The sample points of every CTA, E then H, each in ring order: shared-memory
 // offset (E_x outside it: storage index) with its flags, and ring position.
