@@ -89,9 +89,11 @@ __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)_
 // last ones run, to wait here in turn.  Every thread of a kernel that is
 // launched this way calls it before it touches memory, so a grid past it has
 // all earlier ones behind it.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void grid_order() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  grid_wait();
+  grid_next();
 }
 
 // mbarriers (shared memory, this CTA) and their bounded wait.

@@ -1254,8 +1254,13 @@ __device__ __forceinline__ void d64_digits(long long X, unsigned d[D64_D]) {
 // Twiddles dt exp(i fw t_k) of nk samples as B operands: sub-block, group g,
 // digit s, row n = 2 j + d (frequency 32 g + j), column 2 k + c, the real 2 x 2 form of
 // the complex product.  eb: biased exponent of their common scale (dt's).
-__global__ void __launch_bounds__(256) k_twiddle_d64(const int* __restrict__ tk, int nk, const double* __restrict__ fw,
+// 64 threads a CTA: a few thousand FP64 sincos are bound by the FP64 pipes of
+// the SMs they sit on.  k_dft_d64 starts beside it (samples and digits) and
+// waits for it before its first B: a block of 192 points and 200 frequencies
+// takes 29 us, in sequence and with 256 threads a CTA 34.5.
+__global__ void __launch_bounds__(64) k_twiddle_d64(const int* __restrict__ tk, int nk, const double* __restrict__ fw,
                                                      int nof, double dt, int ngroups, __nv_bfloat16_raw* __restrict__ Bt) {
+  grid_next();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;  // (sub-block, group, frequency, sample)
   const int kk = t % D64_S, j = (t / D64_S) % D64_F, sg = t / (D64_S * D64_F), g = sg % ngroups, iw = g * D64_F + j;
   const int k = sg / ngroups * D64_S + kk;
@@ -1346,7 +1351,6 @@ template <bool FLUX> __global__ void __launch_bounds__(D64_THREADS, 1) k_dft_d64
     mbar_expect_tx(&bar_b, 2u * D64_D * D64_B);
     bulk_g2s(sb, A.Bt + (k * A.ngroups + item % A.ngroups) * (long)(D64_D * D64_B), 2u * D64_D * D64_B, &bar_b);
   };
-  if (tid == 0 && nsteps > 0) load_b(0);
   long have = -1;  // (tile, sub-block) whose digits are in A
   bool go = true;
   for (long item = i0; item < i1 && go; ++item) {
@@ -1403,6 +1407,10 @@ template <bool FLUX> __global__ void __launch_bounds__(D64_THREADS, 1) k_dft_d64
             *(uint4*)(sa + s * D64_A + d64_off(r, 16 * h8 + 8 * h)) = make_uint4(d[s][0], d[s][1], d[s][2], d[s][3]);
         }
         fence_proxy_async();  // the generic-proxy writes of A before the tensor core reads them
+        if (tid == 0 && q == 0) {  // the first twiddles: their kernel may still run, beside everything so far
+          grid_wait();
+          load_b(0);
+        }
         __syncthreads();
       }
       if (tid == 0) {
@@ -3062,7 +3070,7 @@ static D64Args d64_args(iris_engine* E, int nk) {
   A.ngroups = (E->p.nof + D64_F - 1) / D64_F;
   A.eb = std::ilogb(E->p.dt) + 1023;
   A.err = E->d_err;
-  k_twiddle_d64<<<(unsigned)(A.nsb * A.ngroups * D64_F * D64_S / 256), 256, 0, E->st>>>(
+  k_twiddle_d64<<<(unsigned)(A.nsb * A.ngroups * D64_F * D64_S / 64), 64, 0, E->st>>>(
       E->d_tk, nk, E->d_fw, A.nof, E->p.dt, A.ngroups, (__nv_bfloat16_raw*)E->d_wt64);
   return A;
 }
@@ -3076,7 +3084,7 @@ void dft_flush(iris_engine* E) {
   if (E->prec == IRIS_FP64) {
     D64Args A = d64_args(E, nk);
     A.nitems = (E->P + D64_M - 1) / D64_M * A.ngroups;
-    k_dft_d64<false><<<(unsigned)std::min<long>(A.nitems, E->ws_blocks), D64_THREADS, D64_SMEM, E->st>>>(A);
+    launch_ordered_smem(k_dft_d64<false>, (unsigned)std::min<long>(A.nitems, E->ws_blocks), D64_THREADS, D64_SMEM, E->st, A);
     E->fd_zero = false;  // every accumulator of every frequency has been written
   } else if (E->dft_tc) {
     const int ng = (E->p.nof + TC_NW - 1) / TC_NW, nch = (2 * nk + TC_KC - 1) / TC_KC;
@@ -3558,7 +3566,7 @@ int iris::read_flux(iris_engine* E, int set, double* J) {
       A.faces = E->d_faces + 6 * set;
       A.ft = ft;
       A.part = E->d_part;
-      k_dft_d64<true><<<(unsigned)std::min<long>(A.nitems, E->ws_blocks), D64_THREADS, D64_SMEM, E->st>>>(A);
+      launch_ordered_smem(k_dft_d64<true>, (unsigned)std::min<long>(A.nitems, E->ws_blocks), D64_THREADS, D64_SMEM, E->st, A);
     }
     k_flux_sum<<<dim3(p.nof, 6), 256, 0, E->st>>>(E->d_part, ft, E->d_faces + 6 * set, p.nof, scale, E->d_J);
   } else {
