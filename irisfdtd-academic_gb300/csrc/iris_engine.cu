@@ -3270,6 +3270,16 @@ void one_step(iris_engine* E, int it, int left, bool dft) {
   }
 }
 
+int tfsf_alloc(iris_engine* E) {
+  if (E->src.variant == 0) return IRIS_OK;
+  // a span of at most 1024 steps and 8 MB
+  const int ncol = E->p.nx + 2;
+  E->tfv_cap = (int)std::max(1L, std::min(1024L, (8L << 20) / (32L * ncol)));
+  if (cudaMalloc(&E->d_tfv, sizeof(TfsfVal<double>) * (size_t)E->tfv_cap * ncol) == cudaSuccess) return IRIS_OK;
+  cudaGetLastError();
+  return fail(IRIS_ENOMEM, "TF/SF table allocation failed");
+}
+
 // packed: rows of nx+2 cells back to back (no 128-byte alignment of x = 1),
 // for cells whose rows are short; component arrays stay 128-byte aligned.
 int create_engine(const iris_params* pin, const double* fw, bool member, bool z_only, iris_engine** out,
@@ -3395,12 +3405,7 @@ int create_engine(const iris_params* pin, const double* fw, bool member, bool z_
                                     "fewer than 2^31 / 3 cells"));
     if (E->persist && cudaMalloc(&E->d_bar, 64) != cudaSuccess)
       return bail(fail(IRIS_ENOMEM, "barrier allocation failed"));
-    if (!member && E->src.variant != 0) {
-      // TF/SF table of a span: at most 1024 steps and 8 MB
-      E->tfv_cap = (int)std::max(1L, std::min(1024L, (8L << 20) / (32L * (p.nx + 2))));
-      if (cudaMalloc(&E->d_tfv, sizeof(TfsfVal<double>) * (size_t)E->tfv_cap * (p.nx + 2)) != cudaSuccess)
-        return bail(fail(IRIS_ENOMEM, "TF/SF table allocation failed"));
-    }
+    if (!member && (rc = tfsf_alloc(E))) return bail(rc);
   }
   if (E->persist) {
     rc = res_setup(E);
@@ -3710,6 +3715,7 @@ int iris_flux(iris_engine* E, int box, double* J) {
   iris::NvtxRange nvtx_("iris_flux");
   clear_error();
   if (!E || !J || box < 0 || box > 1) return fail(IRIS_EINVAL, "bad argument");
+  if (E->member) return fail(IRIS_EINVAL, "the adjoint state takes no DFT samples");
   CK(cudaSetDevice(E->device));
   if (box >= E->nboxes) box = 0;  // a single box: the second one is the same box
   return read_flux(E, box, J);
@@ -3957,6 +3963,7 @@ int iris_get_plane(iris_engine* E, int which, int axis, int index, int lo1, int 
 int iris_get_fdata(iris_engine* E, int box, int j, double* re, double* im, long* npts) {
   clear_error();
   if (!E || box < 0 || box > 1 || j < 1 || j > 3) return fail(IRIS_EINVAL, "bad argument");
+  if (E->member) return fail(IRIS_EINVAL, "the adjoint state takes no DFT samples");
   CK(cudaSetDevice(E->device));
   if (box >= E->nboxes) box = 0;
   const FaceMap& F = E->fm[box][j - 1];
