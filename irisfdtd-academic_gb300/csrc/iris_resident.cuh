@@ -36,10 +36,16 @@ namespace iris {
 // its step's tag, and the lane that needs it polls for it.  A phase then
 // waits for one store to become visible instead of the CTA's last store, a
 // barrier, a release and the load behind the acquire.  A packet needs one
-// place only: the number it is a function of next is computed, and published
-// back, by the very lane that read it, and the lane that overwrites it has
-// read that (curl E and curl H are transposes of one another).  4x4x512: 5.9 us
-// a step before, 4.4 so; 1x1x400 5.7 and 4.4.
+// place only: the number it is a function of next is published back by the
+// lanes that read it, and the lane that overwrites it has read all of those
+// (curl E and curl H are transposes of one another).  A lane reads the packet
+// of its own part p, or both parts where the row it reads is a Bloch image
+// with a phase, and the two directions across a border agree on which
+// (res_ll_ask); what a complex material needs of the other part comes from the
+// neighbouring lane, so a number's publication follows from the reads of both
+// lanes of its pair, not from their running in step.  The same order keeps a
+// span's last H phase from overwriting ghosts that its first E phase still
+// reads.  4x4x512: 5.9 us a step before, 4.4 so; 1x1x400 5.7 and 4.4.
 //
 // TF/SF.  The H correction is added as the H phase stores (nothing else reads
 // that H in the phase); the E correction of step i is added when step i+1's E
@@ -595,6 +601,12 @@ __device__ __forceinline__ bool res_ll_get(const ulonglong2* const (&q)[4], unsi
   }
   return true;
 }
+// The packets of the number whose parts lie at b that a lane with part p reads
+// (in q, q + 1): both where the row is an image with a phase, else its own.
+__device__ __forceinline__ void res_ll_ask(const ulonglong2** q, const ulonglong2* b, bool image, int p) {
+  q[0] = image ? b : b + p;
+  if (image) q[1] = b + 1;
+}
 // What a phase of a step needs of LL: the tag of what it reads (0: nothing,
 // the first step's E phase reads the state in memory) and of what it
 // publishes, the wait's limit and where a wait that gave up is noted.
@@ -627,21 +639,14 @@ __device__ __forceinline__ void res_e64(const ResArgs<double>& A, const ResView<
   const int i = k == 2 ? 0 : k + 1, j = k == 0 ? 2 : k - 1;
   const double2 *hi = v.h(i), *hj = v.h(j);
   // LL: the packets of component j down axis i and of component i down axis j
-  // (both parts where a phase or a complex material mixes them, else part p)
-  double pk[4];
+  double pk[4] = {};
   if constexpr (LL) {
     if (ll.want) {
       const ulonglong2* q[4] = {};
       auto ask = [&](int ax, int c, int at) {
-        const int gl = ax == 1 ? RF_YG : RF_ZG, im = ax == 1 ? RF_YP : RF_ZP;
-        if (ax == 0 || !(r.fl & gl)) return;
-        const ulonglong2* b = A.ll + 2l * ((3 + c) * cp + gi + (ax == 1 ? r.yo : r.zo));
-        if (CEPS || (r.fl & im)) {
-          q[at] = b;
-          q[at + 1] = b + 1;
-        } else {
-          q[at] = b + p;
-        }
+        if (ax != 0 && (r.fl & (ax == 1 ? RF_YG : RF_ZG)))
+          res_ll_ask(q + at, A.ll + 2l * ((3 + c) * cp + gi + (ax == 1 ? r.yo : r.zo)),
+                     (r.fl & (ax == 1 ? RF_YP : RF_ZP)) != 0, p);
       };
       ask(i, j, 0);
       ask(j, i, 2);
@@ -651,26 +656,22 @@ __device__ __forceinline__ void res_e64(const ResArgs<double>& A, const ResView<
       }
     }
   }
-  // part q of component c one cell down axis ax
-  auto nb = [&](const double2* hc, int c, int ax, int q) {
-    if (ax == 0) return res_ds(hc, li - 1, q);
+  // part p of component c one cell down axis ax
+  auto nb = [&](const double2* hc, int c, int ax) {
+    if (ax == 0) return res_ds(hc, li - 1, p);
     const int off = ax == 1 ? r.yo : r.zo, gl = ax == 1 ? RF_YG : RF_ZG, im = ax == 1 ? RF_YP : RF_ZP;
     if (LL && (r.fl & gl) && ll.want) {
       const double u = c == j ? pk[0] : pk[2], w = c == j ? pk[1] : pk[3];
-      if (r.fl & im) return res_dph(ax == 1 ? a.pym : a.pzm, cx<double>{u, w}, q);
-      return CEPS && q ? w : u;
+      return r.fl & im ? res_dph(ax == 1 ? a.pym : a.pzm, cx<double>{u, w}, p) : u;
     }
     if (r.fl & im) {
       const double2 w = (r.fl & gl) ? __ldcg(a.h + c * cp + gi + off) : hc[li + off];
-      return res_dph(ax == 1 ? a.pym : a.pzm, cx<double>{w.x, w.y}, q);
+      return res_dph(ax == 1 ? a.pym : a.pzm, cx<double>{w.x, w.y}, p);
     }
-    return (r.fl & gl) ? res_dl2(a.h + c * cp, gi + off, q) : res_ds(hc, li + off, q);
-  };
-  auto curl = [&](int q) {
-    return da(ds(ds(res_ds(hj, li, q), nb(hj, j, i, q)), res_ds(hi, li, q)), nb(hi, i, j, q));
+    return (r.fl & gl) ? res_dl2(a.h + c * cp, gi + off, p) : res_ds(hc, li + off, p);
   };
   double e = NC == 5 && k == 0 ? res_dl2(a.e, gi, p) : res_ds(v.e(k), li, p);
-  const double c = curl(p);
+  const double c = da(ds(ds(res_ds(hj, li, p), nb(hj, j, i)), res_ds(hi, li, p)), nb(hi, i, j));
   if ((r.fl & RF_CORR) && k == A.s.cE) {
     const double t = p == 0 ? vE[x].er : vE[x].ei;
     e = A.s.sgn > 0 ? da(e, t) : ds(e, t);
@@ -688,7 +689,8 @@ __device__ __forceinline__ void res_e64(const ResArgs<double>& A, const ResView<
     const int ie = gi - a.hi * (int)g.plane;
     if (CEPS) {
       const double2 w = a.eps_c[ie];
-      const double o = curl(p ^ 1);
+      const cx<double> cc = res_pair(c, p);
+      const double o = p == 0 ? cc.im : cc.re;
       e = axpy_(w.x, c, axpy_(p == 0 ? -w.y : w.y, o, e));
     } else {
       e = axpy_(a.eps_r[ie], c, e);
@@ -717,15 +719,13 @@ __device__ __forceinline__ void res_h64(const ResArgs<double>& A, const ResView<
   const int li = lrow * v.W + x, gi = r.gb + x, cp = (int)g.comp;
   if (!bc_ok(x >= 1 && x <= g.nx && lrow < v.nrows, BC_H_CELL, gi)) return;
   const int i = k == 2 ? 0 : k + 1, j = k == 0 ? 2 : k - 1;
-  double pk[4];
+  double pk[4] = {};
   if constexpr (LL) {
     const ulonglong2* q[4] = {};
     auto ask = [&](int ax, int c, int at) {
-      const int gl = ax == 1 ? RF_YG : RF_ZG, im = ax == 1 ? RF_YP : RF_ZP;
-      if (ax == 0 || !(r.fl & gl)) return;
-      const ulonglong2* b = A.ll + 2l * (c * cp + gi + (ax == 1 ? r.yo : r.zo));
-      q[at] = b + ((r.fl & im) ? 0 : p);
-      if (r.fl & im) q[at + 1] = b + 1;
+      if (ax != 0 && (r.fl & (ax == 1 ? RF_YG : RF_ZG)))
+        res_ll_ask(q + at, A.ll + 2l * (c * cp + gi + (ax == 1 ? r.yo : r.zo)),
+                   (r.fl & (ax == 1 ? RF_YP : RF_ZP)) != 0, p);
     };
     ask(i, j, 0);
     ask(j, i, 2);
