@@ -133,14 +133,19 @@ typedef struct iris_params {
   int graph;          /* 1: step whole DFT blocks (every step sampled) by
                          replaying one captured CUDA graph; results are
                          identical to launch-by-launch stepping            */
-  int dft_kernel;     /* IRIS_DFT_KERNEL_*: FP32 DFT block accumulation    */
+  int dft_kernel;     /* IRIS_DFT_KERNEL_*: DFT block accumulation         */
 } iris_params;
 
-/* ---- FP32 DFT block kernels (iris_params.dft_kernel) ------------------ */
+/* ---- DFT block kernels (iris_params.dft_kernel) ----------------------- */
 #define IRIS_DFT_KERNEL_AUTO 0   /* the engine's choice (tensor cores)      */
-#define IRIS_DFT_KERNEL_CUDA 1   /* FP32 FMA on the CUDA cores              */
-/* tcgen05 tensor cores, TF32 operands split hi + lo (three MMAs per product,
- * FP32-level accuracy), FP32 partial sums in TMEM, FP64 accumulators      */
+/* FMAs on the CUDA cores.  IRIS_FP32: FP32 partial sums over a block;
+ * IRIS_FP64: one sample after another into the FP64 accumulators, in the
+ * reference's order, so the sums do not depend on where a block ends      */
+#define IRIS_DFT_KERNEL_CUDA 1
+/* tcgen05 tensor cores.  IRIS_FP32: TF32 operands split hi + lo (three MMAs
+ * per product, FP32-level accuracy), FP32 partial sums in TMEM, FP64
+ * accumulators; IRIS_FP64: exact integer digit products of a block, added to
+ * the FP64 accumulators with one rounding                                  */
 #define IRIS_DFT_KERNEL_TENSOR 2
 
 /* ---- DFT faces (iris_params.dft_faces) -------------------------------- */

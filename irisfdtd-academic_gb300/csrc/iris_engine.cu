@@ -1170,6 +1170,57 @@ __global__ void __maxnreg__(80) k_dft_ws_commit(WsArgs A) { dft_ws<false>(A); }
 __global__ void __launch_bounds__(WsCfg<true>::THREADS, 1) k_dft_ws_flux(WsArgs A) { dft_ws<true>(A); }
 
 // ---------------------------------------------------------------------------
+// FP64 DFT block on the CUDA cores (IRIS_DFT_KERNEL_CUDA): fdata(p, iw) +=
+// (dt*F_k(p))*exp(i*fw(iw)*t_k) with k in the reference's order
+// (code/dataprocess.f90:143-147), so the sums do not depend on where a block
+// ends; each complex multiply-add as four FP64 FMAs.  The twiddles
+// exp(i*fw*t_k) come from one table a block.  Bound by FP64 issue.
+constexpr int DFT64_WC = 8;
+__global__ void k_twiddle64(const int* __restrict__ tk, int nk, const double* __restrict__ fw, int nof,
+                            double2* __restrict__ W) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= nk * nof) return;
+  const int k = t / nof, j = t % nof;
+  double sn, cs;
+  sincos(dm(fw[j], (double)tk[k]), &sn, &cs);
+  W[t] = make_double2(cs, sn);
+}
+
+__global__ void __launch_bounds__(128) k_dft_fp64(const double2* __restrict__ S, long P, int nk,
+                                                  const double2* __restrict__ W, int nof, int nwc, double dt,
+                                                  double2* __restrict__ fd) {
+  extern __shared__ double2 W64[];  // [nk][WC]
+  // 1-D grid, frequency chunks fastest: the chunks of one point block share its samples in L2
+  const int w0 = (blockIdx.x % nwc) * DFT64_WC;
+  const long pblk = blockIdx.x / nwc;
+  for (int t = threadIdx.x; t < nk * DFT64_WC; t += blockDim.x) {
+    const int k = t / DFT64_WC, j = t % DFT64_WC;
+    W64[t] = w0 + j < nof ? W[(long)k * nof + w0 + j] : make_double2(0.0, 0.0);
+  }
+  __syncthreads();
+  const long p = pblk * blockDim.x + threadIdx.x;
+  if (p >= P) return;
+  const int nw = min(DFT64_WC, nof - w0);
+  double2 acc[DFT64_WC];
+#pragma unroll
+  for (int j = 0; j < DFT64_WC; ++j)
+    if (j < nw) acc[j] = fd[(long)(w0 + j) * P + p];
+  for (int k = 0; k < nk; ++k) {
+    const double2 f = S[(long)k * P + p];
+    const double ar = dm(dt, f.x), ai = dm(dt, f.y);
+#pragma unroll
+    for (int j = 0; j < DFT64_WC; ++j) {
+      const double2 w = W64[k * DFT64_WC + j];
+      acc[j].x = fma(ar, w.x, fma(-ai, w.y, acc[j].x));
+      acc[j].y = fma(ar, w.y, fma(ai, w.x, acc[j].y));
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < DFT64_WC; ++j)
+    if (j < nw) fd[(long)(w0 + j) * P + p] = acc[j];
+}
+
+// ---------------------------------------------------------------------------
 // FP64 DFT block on the tensor cores (tcgen05.mma kind::f16, exact slices).
 //
 // fdata[iw][p] += sum_k F_k(p) dt exp(i fw(iw) t_k) in FP64 is 4 FP64 FMAs a
@@ -3080,12 +3131,19 @@ void dft_flush(iris_engine* E) {
   KTimer tm(E, IRIS_KC_DFT);
   const int nk = E->nslot;
   // the CUDA-core blocks read what they add to (on a failure the samples stay buffered)
-  if (E->prec != IRIS_FP64 && !E->dft_tc && fd_materialise(E)) return;
-  if (E->prec == IRIS_FP64) {
+  if (!E->dft_d64 && !E->dft_tc && fd_materialise(E)) return;
+  if (E->dft_d64) {
     D64Args A = d64_args(E, nk);
     A.nitems = (E->P + D64_M - 1) / D64_M * A.ngroups;
     launch_ordered_smem(k_dft_d64<false>, (unsigned)std::min<long>(A.nitems, E->ws_blocks), D64_THREADS, D64_SMEM, E->st, A);
     E->fd_zero = false;  // every accumulator of every frequency has been written
+  } else if (E->prec == IRIS_FP64) {
+    const int nwc = (E->p.nof + DFT64_WC - 1) / DFT64_WC;
+    const long nblk = (E->P + 127) / 128;
+    double2* W = (double2*)E->d_wt64;
+    k_twiddle64<<<(unsigned)(((long)nk * E->p.nof + 255) / 256), 256, 0, E->st>>>(E->d_tk, nk, E->d_fw, E->p.nof, W);
+    k_dft_fp64<<<(unsigned)(nblk * nwc), 128, (size_t)nk * DFT64_WC * sizeof(double2), E->st>>>(
+        (const double2*)E->S, E->P, nk, W, E->p.nof, nwc, E->p.dt, (double2*)E->fd);
   } else if (E->dft_tc) {
     const int ng = (E->p.nof + TC_NW - 1) / TC_NW, nch = (2 * nk + TC_KC - 1) / TC_KC;
     const long nt = (long)ng * nch * TC_BROWS * TC_KC;
@@ -3177,7 +3235,8 @@ int alloc_dft(iris_engine* E, const FluxFace* faces, int nfaces) {
   CK(cudaMemGetInfo(&freeb, &totb));
   const size_t fd_bytes = (size_t)P * p.nof * sizeof(double2);
   if (fd_bytes > freeb) return fail(IRIS_ENOMEM, "DFT accumulators exceed free device memory");
-  // FP64: at most 256 slots, 32 by default (accumulated 32 at a time).  FP32: up to 512, the default: a block
+  // FP64: at most 256 slots (the CUDA-core block stages K x 8 twiddles in 32 KB
+  // of shared memory), 32 by default (the digit products take 32 at a time).  FP32: up to 512, the default: a block
   // reads and writes the FP64 accumulators once, so a longer block moves
   // fewer accumulator bytes per sample.  The ring takes at most half of the
   // memory left after the accumulators.
@@ -3195,7 +3254,9 @@ int alloc_dft(iris_engine* E, const FluxFace* faces, int nfaces) {
   CK(cudaMalloc(&E->d_fw, sizeof(double) * p.nof));
   CK(cudaMemcpy(E->d_fw, E->fw.data(), sizeof(double) * p.nof, cudaMemcpyHostToDevice));
   if (E->prec == IRIS_FP32) CK(cudaMalloc(&E->d_wt, sizeof(float2) * (size_t)E->K * p.nof));
-  if (E->prec == IRIS_FP64) {
+  E->dft_d64 = E->prec == IRIS_FP64 && p.dft_kernel != IRIS_DFT_KERNEL_CUDA;
+  if (E->prec == IRIS_FP64 && !E->dft_d64) CK(cudaMalloc(&E->d_wt64, sizeof(double2) * (size_t)E->K * p.nof));
+  if (E->dft_d64) {
     CK(cudaMalloc(&E->d_wt64, 2 * (size_t)D64_D * D64_B * ((p.nof + D64_F - 1) / D64_F) * ((E->K + D64_S - 1) / D64_S)));
     CK(cudaFuncSetAttribute(k_dft_d64<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)D64_SMEM));
     CK(cudaFuncSetAttribute(k_dft_d64<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)D64_SMEM));
@@ -3211,7 +3272,7 @@ int alloc_dft(iris_engine* E, const FluxFace* faces, int nfaces) {
     CK(cudaFuncSetAttribute(k_dft_ws_commit, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WS_SMEM));
     CK(cudaFuncSetAttribute(k_dft_ws_flux, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WS_SMEM));
   }
-  if (E->dft_tc || E->prec == IRIS_FP64) {
+  if (E->dft_tc || E->dft_d64) {
     long maxt = 1;
     for (int s = 0; s + 6 <= nfaces; s += 6) maxt = std::max(maxt, (long)flux_tiles(faces + s).start[6]);
     CK(cudaMalloc(&E->d_part, sizeof(double) * 4 * (size_t)maxt * p.nof));
@@ -3563,7 +3624,7 @@ int iris::read_flux(iris_engine* E, int set, double* J) {
       k_dft_ws_flux<<<(unsigned)std::min<long>(A.nitems, E->ws_blocks), WsCfg<true>::THREADS, WS_SMEM, E->st>>>(A);
     }
     k_flux_sum<<<dim3(p.nof, 6), 256, 0, E->st>>>(E->d_part, ft, E->d_faces + 6 * set, p.nof, scale, E->d_J);
-  } else if (E->prec == IRIS_FP64 && E->nslot > 0) {
+  } else if (E->dft_d64 && E->nslot > 0) {
     KTimer tm(E, IRIS_KC_FLUX);
     if (ft.start[6] > 0) {
       D64Args A = d64_args(E, E->nslot);

@@ -83,7 +83,8 @@ struct iris_engine {
   // (fd_materialise)
   bool fd_zero = false;
   float2* d_wt = nullptr;
-  void* d_wt64 = nullptr;  // FP64 mode: B operands of 32 samples (k_twiddle_d64)
+  void* d_wt64 = nullptr;  // FP64 mode: the B operands of a block (k_twiddle_d64), or its twiddles (k_twiddle64)
+  bool dft_d64 = false;    // FP64 block accumulation on the tensor cores
   bool dft_tc = false;     // FP32 block accumulation on the tensor cores
   float* d_wtc = nullptr;  // its B operands (k_twiddle_tc)
   int ws_blocks = 0;       // CTAs of its persistent launches (one per SM)
