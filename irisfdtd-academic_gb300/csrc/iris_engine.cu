@@ -1353,16 +1353,21 @@ struct D64Args {
   int* err;
 };
 
-// The double nearest V 2^e (round half away from zero; 0 below the normal
-// range), formed with integer operations.
+// The double nearest V 2^e (round half away from zero), formed with integer
+// operations.
 __device__ __forceinline__ double d64_value(long long V, int e) {
   if (V == 0) return 0.0;
   unsigned long long m = V < 0 ? 0ull - (unsigned long long)V : (unsigned long long)V;
   const int lz = __clzll((long long)m);
   m <<= lz;
   const int be = 1023 + 63 - lz + e;
-  if (be < 1) return 0.0;
-  if (be > 2045) return V < 0 ? -__longlong_as_double(0x7ff0000000000000ll) : __longlong_as_double(0x7ff0000000000000ll);
+  if (be < 1) {  // below the normal range: a multiple of 2^-1074
+    const int sh = 12 - be;
+    if (sh > 64) return 0.0;
+    const unsigned long long q = (sh < 64 ? m >> sh : 0ull) + ((m >> (sh - 1)) & 1ull);
+    return __longlong_as_double((long long)(q | (V < 0 ? 1ull << 63 : 0ull)));
+  }
+  if (be > 2046) return V < 0 ? -__longlong_as_double(0x7ff0000000000000ll) : __longlong_as_double(0x7ff0000000000000ll);
   const unsigned long long q = (m >> 11) + ((m >> 10) & 1ull);
   return __longlong_as_double((long long)((((unsigned long long)(be - 1)) << 52) + q + (V < 0 ? 1ull << 63 : 0ull)));
 }
