@@ -2784,7 +2784,8 @@ int res_samples(iris_engine* E) {
 // Steps it0 .. it0+n-1 with the persistent kernel: spans that end where the
 // DFT ring fills (its commit runs between launches), after 1024 steps or at
 // the TF/SF table's capacity; before each span k_tfsf_table evaluates its
-// TF/SF corrections.
+// TF/SF corrections.  By default a resident engine takes a span of one step
+// with the split passes.
 template <typename T> int step_persist(iris_engine* E, int it0, int n) {
   const iris_params& p = E->p;
   const int cap = E->src.variant != 0 ? E->tfv_cap : 1024;
@@ -2809,6 +2810,21 @@ template <typename T> int step_persist(iris_engine* E, int it0, int n) {
       const int t = it + span;
       ++span;
       if (E->P > 0 && t >= p.to_fourier && t % p.sample_fourier == 0 && ++samples + E->nslot == E->K) break;
+    }
+    if (E->res && span == 1 && p.stencil == IRIS_STENCIL_DEFAULT) {
+      // a span of one step would load and store the whole resident state around
+      // two phases: the split passes, the same bits, take it (us a call of one
+      // step, resident and split: FP32 4x4x512 28.3 and 16.6, 61x47x203 43.6 and
+      // 27.0, 256x4x768 43.7 and 28.9; FP64 1x1x400 25.4 and 24.1, 4x4x512 28.5
+      // and 25.5, 256x4x340 91.8 and 65.5; two steps: 31.2 and 24.0, 57.0 and
+      // 44.7, 53.9 and 46.5; 32.5 and 42.9, 34.9 and 43.9, 147 and 121)
+      E->tf_end = 0;
+      launch_e<T>(E);
+      launch_h<T>(E);
+      finish_step<T>(E, it, 1, nullptr, samples > 0);
+      E->tf_end = 0;
+      ++it;
+      continue;
     }
     TinyArgs<T> A{};
     A.a = field_args<T>(E);
