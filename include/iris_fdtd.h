@@ -389,6 +389,15 @@ int iris_timing_read(iris_engine* eng, double* region_ms, double* kernel_ms, lon
  * material flag, [5] number of DFT boxes, [6] DFT samples buffered and not
  * yet accumulated into fdata (info: 7 entries). */
 int iris_info(const iris_engine* eng, long* info);
+/* How the engine steps (info: 10 entries): info[0] IRIS_STENCIL_SPLIT, FUSED,
+ * STREAM or PERSISTENT; info[1] its form.  FUSED: 1 staged tiles, then [2..5]
+ * their cells in x and y and their number across x and y outside the UPML
+ * slabs, [6..9] the same in them; 0 a column a thread (offsets past 32 bits).
+ * PERSISTENT: 0 grid-wide barriers, 1 resident in shared memory with flags
+ * between neighbours, 2 with packets; 1 and 2: [2] CTAs, [3] components of E
+ * and H in shared memory, [4] D and B there, [5] warps take runs of 32 cells.
+ * Entries without a meaning are 0. */
+int iris_stepping(const iris_engine* eng, long* info);
 /* Bounds-check record of the process's kernels.  Returns 1 when the library
  * was built with bounds checks (libiris_fdtd_bc.so, -DIRIS_BOUNDS_CHECK), 0
  * otherwise; *first receives the first out-of-range access any kernel met

@@ -291,6 +291,18 @@ class Engine:
         return dict(dft_points=a[0], dft_block=a[1], bytes_per_complex=a[2], comp_elems=a[3],
                     complex_material=bool(a[4]), boxes=a[5], dft_buffered=a[6])
 
+    def stepping(self) -> dict:
+        """How the engine steps (iris_stepping): its stencil and form, and the staged
+        tiles of the fused pass or the resident kernel's layout."""
+        a = (ctypes.c_long * 10)()
+        check(self.L.iris_stepping(self.h, a), "iris_stepping")
+        d = dict(stencil=a[0], form=a[1])
+        if a[0] == STENCIL_FUSED and a[1]:
+            d.update(tile=(a[2], a[3]), tiles=(a[4], a[5]), slab_tile=(a[6], a[7]), slab_tiles=(a[8], a[9]))
+        elif a[0] == STENCIL_PERSISTENT and a[1]:
+            d.update(ctas=a[2], components=a[3], upml_resident=bool(a[4]), runs=bool(a[5]))
+        return d
+
     def dft_commit(self):
         """Accumulate the buffered DFT samples into fdata now (iris_dft_commit)."""
         check(self.L.iris_dft_commit(self.h), "iris_dft_commit")

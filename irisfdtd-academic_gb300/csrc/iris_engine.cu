@@ -4138,6 +4138,28 @@ int iris_info(const iris_engine* E, long* info) {
   return IRIS_OK;
 }
 
+int iris_stepping(const iris_engine* E, long* info) {
+  if (!E || !info) return fail(IRIS_EINVAL, "bad argument");
+  for (int i = 0; i < 10; ++i) info[i] = 0;
+  if (E->persist) {
+    info[0] = IRIS_STENCIL_PERSISTENT;
+    if (!E->res) return IRIS_OK;
+    info[1] = E->res_ll ? 2 : 1;
+    const long v[] = {E->res_blocks, E->res_nc, E->res_db, E->res_runs};
+    std::copy(v, v + 4, info + 2);
+  } else if (E->fused) {
+    info[0] = IRIS_STENCIL_FUSED;
+    if (E->mshape.id < 0) return IRIS_OK;
+    info[1] = 1;
+    const MarchShape &m = E->mshape, &q = E->sshape;
+    const long v[] = {m.w, m.r, m.tx, m.ty, q.w, q.r, q.tx, q.ty};
+    std::copy(v, v + 8, info + 2);
+  } else {
+    info[0] = E->stream && !E->eps_complex ? IRIS_STENCIL_STREAM : IRIS_STENCIL_SPLIT;
+  }
+  return IRIS_OK;
+}
+
 int iris_bounds_check(unsigned long long* first) {
   clear_error();
   if (!first) return fail(IRIS_EINVAL, "bad argument");

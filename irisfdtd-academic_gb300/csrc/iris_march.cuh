@@ -479,7 +479,7 @@ template <int W, int R> using SlabTile = MarchTile<W, R, MS_T, true>;
 constexpr int SLAB_MAX_SMEM = std::max({IRIS_SLAB_SHAPES(IRIS_SLAB_SMEM) 0});
 #undef IRIS_SLAB_SMEM
 struct MarchShape {
-  int id = -1, tx = 0, ty = 0;  // id < 0: none
+  int id = -1, w = 0, r = 0, tx = 0, ty = 0;  // id < 0: none; cells of a tile, tiles of the plane
   size_t smem = 0;
 };
 inline MarchShape march_shape(int nx, int ny) {
@@ -491,7 +491,7 @@ inline MarchShape march_shape(int nx, int ny) {
     const double c = (double)tx * ty * (W + 24) * (R + 1.5);            \
     if (c < cost) {                                                     \
       cost = c;                                                         \
-      best.id = ID, best.tx = tx, best.ty = ty;                         \
+      best.id = ID, best.w = W, best.r = R, best.tx = tx, best.ty = ty;                        \
       best.smem = MarchTile<W, R>::SMEM;                                \
     }                                                                   \
   }
@@ -508,7 +508,7 @@ inline MarchShape slab_shape(int nx, int ny) {
     const double c = (double)tx * ty * (W + 24) * (R + 1.5);            \
     if (c < cost) {                                                     \
       cost = c;                                                         \
-      best.id = ID, best.tx = tx, best.ty = ty;                         \
+      best.id = ID, best.w = W, best.r = R, best.tx = tx, best.ty = ty;                        \
       best.smem = SlabTile<W, R>::SMEM;                                 \
     }                                                                   \
   }

@@ -116,7 +116,7 @@ EXPORTS = [
     "iris_dft_commit", "iris_material_spheres", "iris_material_pattern", "iris_material_design",
     "iris_get_material", "iris_batch_material_pattern", "iris_write_scatt", "iris_get_field", "iris_set_field", "iris_get_pml", "iris_set_pml",
     "iris_get_field_c", "iris_set_field_c", "iris_get_pml_c", "iris_set_pml_c",
-    "iris_get_fdata", "iris_get_plane", "iris_get_plane_c", "iris_apply", "iris_run_input", "iris_timing", "iris_timing_read", "iris_info",
+    "iris_get_fdata", "iris_get_plane", "iris_get_plane_c", "iris_apply", "iris_run_input", "iris_timing", "iris_timing_read", "iris_info", "iris_stepping",
     "iris_bounds_check",
     "iris_dft_block_noalloc", "iris_batch_create", "iris_batch_destroy", "iris_batch_set_material",
     "iris_batch_step", "iris_batch_flux", "iris_batch_dft_commit", "iris_batch_get_field", "iris_batch_tune",
@@ -179,6 +179,7 @@ def lib():
     L.iris_timing.argtypes = [vp, ip]
     L.iris_timing_read.argtypes = [vp, dp, dp, ctypes.POINTER(ctypes.c_long)]
     L.iris_info.argtypes = [vp, ctypes.POINTER(ctypes.c_long)]
+    L.iris_stepping.argtypes = [vp, ctypes.POINTER(ctypes.c_long)]
     L.iris_bounds_check.argtypes = [ctypes.POINTER(ctypes.c_ulonglong)]
     L.iris_dft_block_noalloc.argtypes = [vp, ip, ctypes.c_long, ip, ip, vp, ip, ctypes.c_double, vp, vp]
     lp = ctypes.POINTER(ctypes.c_long)
