@@ -274,8 +274,9 @@ int iris_sync(iris_engine* eng);
  * major: the Jabs array of scattering_fourier_out
  * (code/dataprocess.f90:243-277), eps0*Q/(2 dt) included.  Returns
  * IRIS_ENAN if any value is not finite.  Every sample taken so far counts;
- * the samples still buffered are added on the fly and stay buffered (except
- * with IRIS_DFT_KERNEL_CUDA), so a flux read changes no state.
+ * the samples still buffered are added on the fly and stay buffered, except
+ * with IRIS_DFT_KERNEL_CUDA and, in IRIS_FP64, when at most three are: those
+ * are accumulated first.
  */
 int iris_flux(iris_engine* eng, int box, double* J);
 

@@ -1254,6 +1254,14 @@ __global__ void __launch_bounds__(128) k_dft_fp64(const double2* __restrict__ S,
 constexpr int D64_M = 128, D64_F = 32, D64_N = 2 * D64_F, D64_S = 32, D64_K = 2 * D64_S, D64_D = 7, D64_O = 8;
 constexpr int D64_A = D64_M * D64_K, D64_B = D64_N * D64_K;  // elements of one digit plane
 constexpr int D64_THREADS = 512;
+// Up to so many samples are accumulated one after another by k_dft_fp64 instead
+// (a digit block costs about the same for 1 sample as for 8), by a flux read
+// too, which otherwise forms a block's products anew each time.  us a call of
+// n steps and a flux read, n = 1, 3, 4, digits and FMAs: 128x128x160 with every
+// face pair at 128 frequencies 2395, 3361, 3525 and 1141, 2915, 3798; z planes at
+// 16 frequencies 599, 1305, 1626 and 461, 1184, 1547; 4x4x512 110, 117, 119 and
+// 88, 100, 100.
+constexpr int D64_FEW = 3;
 constexpr size_t D64_SMEM = 2 * (size_t)D64_D * (D64_A + D64_B);
 
 // Offset of element (row r, k) of a K-major, unswizzled bf16 operand of D64_K
@@ -3152,8 +3160,9 @@ void dft_flush(iris_engine* E) {
   KTimer tm(E, IRIS_KC_DFT);
   const int nk = E->nslot;
   // the CUDA-core blocks read what they add to (on a failure the samples stay buffered)
-  if (!E->dft_d64 && !E->dft_tc && fd_materialise(E)) return;
-  if (E->dft_d64) {
+  const bool d64 = E->dft_d64 && nk > D64_FEW;
+  if (!d64 && !E->dft_tc && fd_materialise(E)) return;
+  if (d64) {
     D64Args A = d64_args(E, nk);
     A.nitems = (E->P + D64_M - 1) / D64_M * A.ngroups;
     launch_ordered_smem(k_dft_d64<false>, (unsigned)std::min<long>(A.nitems, E->ws_blocks), D64_THREADS, D64_SMEM, E->st, A);
@@ -3609,9 +3618,10 @@ static int stream_status(iris_engine* E) {
 // The flux of one face set.  On the tensor cores: over the accumulators plus
 // the samples still in the ring, which stay there (FP32: k_twiddle_tc for the
 // pending samples, k_dft_ws_flux, k_flux_sum; FP64: k_twiddle_d64, k_dft_d64,
-// k_flux_sum, or k_flux when none are pending).  A flux read so never splits a
-// block of samples, whose sums round per block.  On the CUDA cores the ring is
-// committed first and k_flux reads the accumulators.
+// k_flux_sum).  A flux read so never splits a block of samples, whose sums
+// round per block.  On the CUDA cores, and for at most D64_FEW samples in FP64,
+// the ring is committed first (sample by sample in FP64: its sums do not
+// depend on when) and k_flux reads the accumulators.
 int iris::read_flux(iris_engine* E, int set, double* J) {
   const iris_params& p = E->p;
   const double scale = p.eps0 * p.Q / (2.0 * p.dt);
@@ -3645,7 +3655,7 @@ int iris::read_flux(iris_engine* E, int set, double* J) {
       k_dft_ws_flux<<<(unsigned)std::min<long>(A.nitems, E->ws_blocks), WsCfg<true>::THREADS, WS_SMEM, E->st>>>(A);
     }
     k_flux_sum<<<dim3(p.nof, 6), 256, 0, E->st>>>(E->d_part, ft, E->d_faces + 6 * set, p.nof, scale, E->d_J);
-  } else if (E->dft_d64 && E->nslot > 0) {
+  } else if (E->dft_d64 && E->nslot > D64_FEW) {
     KTimer tm(E, IRIS_KC_FLUX);
     if (ft.start[6] > 0) {
       D64Args A = d64_args(E, E->nslot);
