@@ -883,7 +883,7 @@ int iris_adjoint_create(const iris_params* pin, const double* fw, const int desi
   if (rc) return bail(rc);
   q.stencil = IRIS_STENCIL_SPLIT;
   rc = create_engine(&q, fw, true, true, &J->A);
-  if (!rc) rc = tfsf_alloc(J->A);  // callers may step it (iris_adjoint_engine)
+  if (!rc) rc = tfsf_alloc(J->A, 16);  // callers may step it (iris_adjoint_engine)
   if (rc) return bail(rc);
   J->A->P = 0;  // it has no DFT buffers
   iris_engine* F = J->F;

@@ -2593,22 +2593,23 @@ int res_partition(const iris_params& p, int G, double w, std::vector<ResCta>& ou
     out[c].r1 = (int)r;
     widest = std::max(widest, out[c].r1 - out[c].r0);
   }
-  // neighbours: the owners of the ny rows before and after, cyclically
+  return widest;
+}
+
+// The CTAs' neighbours: the owners of the ny rows before and after, cyclically.
+void res_neighbours(const iris_params& p, std::vector<ResCta>& out) {
+  const int G = (int)out.size(), R = p.ny * p.nz;
   std::vector<int> owner(R);
-  for (int c = 0; c < G; ++c)
-    for (int q = out[c].r0; q < out[c].r1; ++q) owner[q] = c;
+  for (int c = 0; c < G; ++c) std::fill(owner.begin() + out[c].r0, owner.begin() + out[c].r1, c);
+  // the rows 1 .. ny away have owners in order, the farthest row the farthest (no
+  // CTA owns the R - ny rows, three quarters at least, that lead round to itself)
+  auto at = [&](int r) { return owner[r < 0 ? r + R : r >= R ? r - R : r]; };
   for (int c = 0; c < G; ++c) {
-    int before = 0, after = 0;
-    for (long d = 1; d <= p.ny; ++d) {
-      const int lo = owner[((out[c].r0 - d) % R + R) % R], hi = owner[(out[c].r1 - 1 + d) % R];
-      before = std::max(before, ((c - lo) % G + G) % G);
-      after = std::max(after, ((hi - c) % G + G) % G);
-    }
+    const int before = (c - at(out[c].r0 - p.ny) + G) % G, after = (at(out[c].r1 - 1 + p.ny) - c + G) % G;
     const int n = std::min(G - 1, before + after);
-    out[c].nb0 = n == G - 1 ? (c + 1) % G : ((c - before) % G + G) % G;
+    out[c].nb0 = n == G - 1 ? (c + 1) % G : (c - before + G) % G;
     out[c].nbn = n == G - 1 ? n : n + 1;  // the CTA itself lies between and has always arrived
   }
-  return widest;
 }
 
 // Whether a persistent engine's state fits in shared memory and its TF/SF
@@ -2676,6 +2677,7 @@ int res_setup(iris_engine* E) {
     fits = true;
   }
   if (!fits) return IRIS_OK;
+  res_neighbours(p, E->res_cta);
   E->res_blocks = G;
   E->res_src = q;
   for (int cplx = 0; cplx < 2; ++cplx) {
@@ -3361,11 +3363,10 @@ void one_step(iris_engine* E, int it, int left, bool dft) {
   }
 }
 
-int tfsf_alloc(iris_engine* E) {
+int tfsf_alloc(iris_engine* E, int steps) {
   if (E->src.variant == 0) return IRIS_OK;
-  // a span of at most 1024 steps and 8 MB
   const int ncol = E->p.nx + 2;
-  E->tfv_cap = (int)std::max(1L, std::min(1024L, (8L << 20) / (32L * ncol)));
+  E->tfv_cap = (int)std::max(1L, std::min<long>(steps, (8L << 20) / (32L * ncol)));
   if (cudaMalloc(&E->d_tfv, sizeof(TfsfVal<double>) * (size_t)E->tfv_cap * ncol) == cudaSuccess) return IRIS_OK;
   cudaGetLastError();
   return fail(IRIS_ENOMEM, "TF/SF table allocation failed");
@@ -3496,7 +3497,7 @@ int create_engine(const iris_params* pin, const double* fw, bool member, bool z_
                                     "fewer than 2^31 / 3 cells"));
     if (E->persist && cudaMalloc(&E->d_bar, 64) != cudaSuccess)
       return bail(fail(IRIS_ENOMEM, "barrier allocation failed"));
-    if (!member && (rc = tfsf_alloc(E))) return bail(rc);
+    if (!member && (rc = tfsf_alloc(E, 1024))) return bail(rc);
   }
   if (E->persist) {
     rc = res_setup(E);

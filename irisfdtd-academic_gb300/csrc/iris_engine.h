@@ -245,9 +245,10 @@ inline MarchSlabArgs march_slab_args(const iris_engine* E) {
 int create_engine(const iris_params* pin, const double* fw, bool member, bool z_only, iris_engine** out,
                   bool packed = false);
 void free_engine(iris_engine* E);
-// The TF/SF table of an engine that steps by itself (iris_step, iris_apply):
-// create_engine does this but for members, whose corrections the batch makes.
-int tfsf_alloc(iris_engine* E);
+// The TF/SF table, of at most so many steps and 8 MB, of an engine that steps by
+// itself (iris_step, iris_apply): create_engine does this but for members, whose
+// corrections the batch makes.
+int tfsf_alloc(iris_engine* E, int steps);
 // DFT buffers for E->P sample points and nfaces flux faces.
 int alloc_dft(iris_engine* E, const FluxFace* faces, int nfaces);
 // Accumulate the sample ring into fdata (one block kernel pass).
