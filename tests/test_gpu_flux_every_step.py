@@ -51,3 +51,19 @@ def test_flux_after_every_call(iris, tmp_path, nx, ny, nof, calls):
         assert np.all(np.abs(J[side] - want[side]) <= 4 * n * n * 2.0 ** -51 * np.sqrt(n) * size.max())
     for x in engines:
         x.close()
+
+
+@pytest.mark.parametrize("block", [1, 3])
+def test_short_blocks_replayed_from_a_graph(iris, tmp_path, block):
+    w = cfg.Workload("d", 13, 9, 60, 4, 57, 25, 8, 2.25, 0, 9, (1, 13, 1, 9, 7, 53), 20, 40)
+    p, fw, _ = iris.setparam(cfg.write_input(str(tmp_path / "in.dat"), w))
+    out = []
+    for graph in (False, True):
+        e = iris.Engine(p, fw, precision=iris.FP64, stencil=iris.STENCIL_SPLIT, dft_block=block, graph=graph)
+        e.step(150, 3 * block)  # the first commit is recorded, the others replay it
+        e.step(150 + 3 * block, 2)
+        out.append([e.get_fdata(0, j) for j in (1, 2, 3)] + [e.flux(0), e.get_field(iris.E)])
+        e.close()
+    assert np.any(out[0][0])
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
