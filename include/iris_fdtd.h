@@ -40,12 +40,15 @@ extern "C" {
 #define IRIS_ENODEV (-8)   /* no CUDA device                                 */
 
 /* ---- precision modes ------------------------------------------------ */
-/* FP64 fields, operations in the reference's order (parity mode); FP64 DFT,
- * a block's partial sums formed to 2^-56 of the point's largest sample and
- * added to fdata with one rounding.                                        */
+/* FP64 fields, operations in the reference's order (parity mode), a product
+ * rounded together with the one sum it goes into; FP64 DFT, a block's partial
+ * sums formed to 2^-56 of the power of two above the point's largest sample
+ * and added to fdata with one rounding (up to three samples, or any number
+ * with IRIS_DFT_KERNEL_CUDA: one after another).                           */
 #define IRIS_FP64 0
-/* FP32 fields; TF/SF incident field in FP64; DFT partial sums over a block
- * of K samples in FP32 with FP64-exact twiddles, accumulated in FP64.     */
+/* FP32 fields; TF/SF incident field evaluated in FP64 and added as two floats
+ * (48 bits); DFT partial sums over a block of K samples in FP32 with
+ * FP64-exact twiddles, accumulated in double-float pairs.                  */
 #define IRIS_FP32 1
 
 /* ---- single operator groups (iris_apply) ----------------------------- */
@@ -172,8 +175,9 @@ typedef struct iris_params {
 #define IRIS_STENCIL_STREAM 3
 /* small grids: one cooperative launch runs a span of whole steps (E, H,
  * TF/SF, DFT sample), the state in shared memory where it fits, the passes
- * separated by flags between neighbours or by grid-wide barriers; the split
- * passes' arithmetic, so the same results bit for bit.  The default for
+ * separated by flags or packets between neighbours or by grid-wide barriers;
+ * the split passes' arithmetic, so the same results bit for bit (by default
+ * they take spans of one step where the state is resident).  The default for
  * grids of at most IRIS_PERSISTENT_MAX_CELLS cells in IRIS_FP64, or
  * IRIS_PERSISTENT_MAX_CELLS_FP32 in IRIS_FP32, that it is estimated to step
  * faster than the split passes (in effect those that fit in shared memory, up
