@@ -405,12 +405,13 @@ __global__ void __launch_bounds__(128) k_tfsf_table(SrcArgs s, int it0, const in
 }
 
 // One step's corrections, row: its table row.  One thread a cell of the
-// corrected planes (latency only: two reads and writes of a value each).
+// corrected planes (latency only: two reads and writes of a value each), tiles
+// of 64 x 4, tx across (all in x: a plane may have more rows than grid.y tiles).
 template <typename T>
 __global__ void __launch_bounds__(256) k_tfsf(typename V2<T>::t* e, typename V2<T>::t* h, Geo g, SrcArgs s,
-                                              const TfsfVal<T>* __restrict__ row) {
+                                              const TfsfVal<T>* __restrict__ row, unsigned tx) {
   grid_order();
-  const int ix = blockIdx.x * 64 + threadIdx.x, iy = blockIdx.y * 4 + threadIdx.y;
+  const int ix = (int)(blockIdx.x % tx * 64 + threadIdx.x), iy = (int)(blockIdx.x / tx * 4 + threadIdx.y);
   if (ix <= s.nx + 1 && iy <= s.ny + 1) tfsf_apply<T>(e, h, g, s, ix, iy, row[ix]);
 }
 
@@ -2383,8 +2384,9 @@ template <typename T> void launch_tfsf(iris_engine* E, int it, int left, const i
   KTimer tm(E, IRIS_KC_TFSF);
   using V = typename V2<T>::t;
   const TfsfVal<T>* row = tfsf_row<T>(E, it, left, itp);
-  const dim3 grd((unsigned)((E->p.nx + 2 + 63) / 64), (unsigned)((E->p.ny + 2 + 3) / 4));
-  launch_ordered(k_tfsf<T>, grd, dim3(64, 4), E->st, (V*)E->e, (V*)E->h, E->g, E->src, row);
+  const unsigned tx = (unsigned)((E->p.nx + 2 + 63) / 64);
+  launch_ordered(k_tfsf<T>, tx * (unsigned)((E->p.ny + 2 + 3) / 4), dim3(64, 4), E->st, (V*)E->e, (V*)E->h, E->g, E->src,
+                 row, tx);
 }
 
 template <typename T> void dft_sample(iris_engine* E, int t, const int* tp = nullptr) {

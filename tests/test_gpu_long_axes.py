@@ -1,0 +1,35 @@
+"""Grids with more rows or planes than 65535 tiles: what a launch maps to grid.y or
+grid.z must still fit.  A column of cells long in y (the TF/SF corrections of
+unsampled steps are a launch of their own) against the persistent kernel, whose
+launch does not depend on the grid's shape."""
+import importlib
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+cfg = importlib.import_module("irisfdtd-academic_gb300.configs")
+
+
+def workload(iris, tmp_path, nx, ny, nz, pml, zi, nof=2):
+    w = cfg.Workload("long", nx, ny, nz, pml, nz + 1 - pml, pml + 2, 2, 2.25, 0, zi, (1, nx, 1, ny, pml + 1, nz - pml), nof, 9)
+    p, fw, _ = iris.setparam(cfg.write_input(str(tmp_path / "in.dat"), w, i_pol=1 if nx == 1 else 2, sample_fourier=4))
+    p.dft_faces = iris.DFT_Z
+    return p, fw
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_rows_past_65535_correction_tiles(iris, tmp_path, precision):
+    p, fw = workload(iris, tmp_path, 1, 263000, 8, 2, 4)
+    out = []
+    for st in (iris.STENCIL_SPLIT, iris.STENCIL_PERSISTENT, iris.STENCIL_DEFAULT):
+        e = iris.Engine(p, fw, precision=precision, stencil=st)
+        e.step(150, 7)
+        e.tfsf(160)
+        e.sync()
+        out.append([e.get_plane(f, 1, 1, (0, p.ny + 1), (0, p.nz + 1)) for f in (iris.E, iris.H)] + [e.flux(0)])
+        e.close()
+    assert np.any(out[0][0][4, 262900:]) and np.any(out[0][2])
+    for o in out[1:]:
+        for a, b in zip(out[0], o):
+            assert np.array_equal(a, b)
