@@ -397,7 +397,8 @@ int iris_info(const iris_engine* eng, long* info);
 /* How the engine steps (info: 10 entries): info[0] IRIS_STENCIL_SPLIT, FUSED,
  * STREAM or PERSISTENT; info[1] its form.  FUSED: 1 staged tiles, then [2..5]
  * their cells in x and y and their number across x and y outside the UPML
- * slabs, [6..9] the same in them; 0 a column a thread (offsets past 32 bits).
+ * slabs, [6..9] the same in them; 0 unstaged columns (offsets past 32 bits, or
+ * more than 65535 rows of tiles).
  * PERSISTENT: 0 grid-wide barriers, 1 resident in shared memory with flags
  * between neighbours, 2 with packets; 1 and 2: [2] CTAs, [3] components of E
  * and H in shared memory, [4] D and B there, [5] warps take runs of 32 cells.

@@ -729,7 +729,9 @@ void adj_setup_march(iris_adjoint* J) {
   iris_engine* S = J->A;
   const iris_params& p = J->F->p;
   if (J->F->prec != IRIS_FP32 || 3 * S->g.comp >= (1L << 31) || p.pmlzf - 2 < p.pmlzi + 2) return;
-  S->mshape = march_shape(p.nx, p.ny);
+  const MarchShape ms = march_shape(p.nx, p.ny);
+  if (ms.ty > MR_MAX_ROWS) return;
+  S->mshape = ms;
   int lo = 0, hi = 0;
   cudaDeviceGetStreamPriorityRange(&lo, &hi);
   J->marched = cudaMalloc(&S->e2, J->fbytes) == cudaSuccess && cudaMalloc(&S->h2, J->fbytes) == cudaSuccess &&

@@ -3535,11 +3535,12 @@ int create_engine(const iris_params* pin, const double* fw, bool member, bool z_
     // z chunks: planes pmlzi+1 .. pmlzf-2 (the last chunk's extra plane,
     // whose E' its H' needs, is then still outside the slabs) by the kernel
     // without slab code, the slabs with the plane next to each by the other;
-    // staged where 32-bit offsets reach
-    const bool staged = 3 * g.comp < (1L << 31);
+    // staged where 32-bit offsets and a launch's tile rows reach
+    const MarchShape ms = march_shape(p.nx, p.ny), ss = slab_shape(p.nx, p.ny);
+    const bool staged = 3 * g.comp < (1L << 31) && ms.ty <= MR_MAX_ROWS && ss.ty <= MR_MAX_ROWS;
     if (staged) {
-      E->mshape = march_shape(p.nx, p.ny);
-      E->sshape = slab_shape(p.nx, p.ny);
+      E->mshape = ms;
+      E->sshape = ss;
       for (bool c : {false, true})
         if (cudaFuncSetAttribute((const void*)march_kernel(E->mshape.id, c), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)E->mshape.smem) != cudaSuccess ||
