@@ -368,12 +368,13 @@ int iris_run_input(const char* dir, int precision);
 /* Kernel classes timed by iris_timing / iris_timing_read. */
 #define IRIS_KC_E 0      /* E update (e_fdtd + UPML-E + Bloch max)        */
 #define IRIS_KC_H 1      /* H update (h_fdtd + UPML-H + Bloch min)        */
-#define IRIS_KC_TFSF 2   /* TF/SF source                                  */
-#define IRIS_KC_GATHER 3 /* DFT face sample gather                        */
+#define IRIS_KC_TFSF 2   /* TF/SF source (launches of its own)            */
+#define IRIS_KC_GATHER 3 /* DFT face sample gather, with the TF/SF source */
+                         /* where they share a launch                     */
 #define IRIS_KC_DFT 4    /* DFT block accumulation (and its twiddles)     */
 #define IRIS_KC_FLUX 5   /* flux reduction                                */
 #define IRIS_KC_FUSED 6  /* fused E+H pass (TF/SF and the DFT sample      */
-                         /* follow as their own kernels)                  */
+                         /* follow as a kernel or two of their own)       */
 #define IRIS_KC_PERSIST 7 /* persistent kernel: a span of whole steps     */
 #define IRIS_NKC 8
 
@@ -385,9 +386,9 @@ int iris_run_input(const char* dir, int precision);
 int iris_timing(iris_engine* eng, int enable);
 /* End the region: its device time, and per kernel class the summed device
  * time (ms) and the number of timed entries (arrays of IRIS_NKC, either may
- * be NULL): one per launch, except the plain engine's IRIS_KC_FUSED (one
- * per step) and the batch's flat work lists (one per E or H pass of two
- * launches). */
+ * be NULL): one per launch, except IRIS_KC_FUSED (one per step), the batch's
+ * flat work lists (one per E or H pass of two launches) and the TF/SF table,
+ * which is part of the entry that needs it. */
 int iris_timing_read(iris_engine* eng, double* region_ms, double* kernel_ms, long* launches);
 /* Sizes: info[0] DFT sample points, [1] DFT block length K, [2] bytes per
  * stored complex value, [3] elements per field component, [4] complex
