@@ -732,7 +732,7 @@ template <typename T> int batch_step_t(iris_batch* B, int it0, int n) {
   int it = it0;
   while (it < it0 + n) {
     if (graph_ready(M, it, it0 + n - it)) {
-      int rc = graph_block(M, it, [&] {
+      int rc = graph_block(M, it, B->parity, [&] {
         B->tf_end = 0;
         for (int j = 0; j < M->K; ++j) batch_one_step<T>(B, j, M->K - j, M->d_it, true);
       });

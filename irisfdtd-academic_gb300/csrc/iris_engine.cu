@@ -2528,7 +2528,7 @@ int step_fused(iris_engine* E, int it0, int n) {
   int it = it0;
   while (it < it0 + n) {
     if (graph_ready(E, it, it0 + n - it)) {
-      int rc = graph_block(E, it, [&] {
+      int rc = graph_block(E, it, E->e > E->e2, [&] {
         E->tf_end = 0;
         for (int j = 0; j < E->K; ++j) fused_one(E, j, E->K - j, E->d_it, true);
       });
@@ -2549,7 +2549,7 @@ template <typename T> int step_t(iris_engine* E, int it0, int n) {
   int it = it0;
   while (it < it0 + n) {
     if (graph_ready(E, it, it0 + n - it)) {
-      int rc = graph_block(E, it, [&] {
+      int rc = graph_block(E, it, 0, [&] {
         E->tf_end = 0;
         for (int j = 0; j < E->K; ++j) {
           launch_e<T>(E);
@@ -3230,21 +3230,26 @@ bool graph_ready(const iris_engine* E, int it, int left) {
 }
 
 void graph_reset(iris_engine* E) {
-  if (E->gexec) cudaGraphExecDestroy(E->gexec);
-  E->gexec = nullptr;
+  for (cudaGraphExec_t& g : E->gexec) {
+    if (g) cudaGraphExecDestroy(g);
+    g = nullptr;
+  }
 }
 
 // Steps it .. it+K-1 from the engine's graph of one DFT block (captured on
 // first use from record(), which issues the K steps with step offsets
 // 0 .. K-1 relative to the device-resident base d_it, the block's sample
-// flush, and the base's advance by K).
-int graph_block(iris_engine* E, int it, const std::function<void()>& record) {
+// flush, and the base's advance by K).  set: which of two buffer sets is current
+// (the fused passes'; single steps between blocks may leave either), whose
+// pointers the capture holds: each set has its own graph.
+int graph_block(iris_engine* E, int it, int set, const std::function<void()>& record) {
+  cudaGraphExec_t& gexec = E->gexec[set];
   if (!E->d_it) {
     CK(cudaMalloc(&E->d_it, sizeof(int)));
     E->dev_it = -1;
   }
   if (E->dev_it != it) k_set_int<<<1, 1, 0, E->st>>>(E->d_it, it);
-  if (!E->gexec) {
+  if (!gexec) {
     // the captured commit is replayed for every block: it must read the sums
     if (int rc = fd_materialise(E)) return rc;
     cudaGraph_t gr = nullptr;
@@ -3253,14 +3258,14 @@ int graph_block(iris_engine* E, int it, const std::function<void()>& record) {
     k_add_int<<<1, 1, 0, E->st>>>(E->d_it, E->K);
     const cudaError_t ec = cudaStreamEndCapture(E->st, &gr);
     if (ec != cudaSuccess) return fail(IRIS_ECUDA, std::string("graph capture: ") + cudaGetErrorString(ec));
-    const cudaError_t ei = cudaGraphInstantiate(&E->gexec, gr, 0);
+    const cudaError_t ei = cudaGraphInstantiate(&gexec, gr, 0);
     cudaGraphDestroy(gr);
     if (ei != cudaSuccess) {
-      E->gexec = nullptr;
+      gexec = nullptr;
       return fail(IRIS_ECUDA, std::string("graph instantiation: ") + cudaGetErrorString(ei));
     }
   }
-  CK(cudaGraphLaunch(E->gexec, E->st));
+  CK(cudaGraphLaunch(gexec, E->st));
   E->dev_it = it + E->K;
   return IRIS_OK;
 }

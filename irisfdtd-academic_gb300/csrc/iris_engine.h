@@ -115,7 +115,7 @@ struct iris_engine {
   cudaEvent_t fz_fork = nullptr, fz_join = nullptr;
   // CUDA graph of one DFT block of steps (iris_params.graph): d_it holds the
   // step base the captured kernels add to their offsets, dev_it its value
-  cudaGraphExec_t gexec = nullptr;
+  cudaGraphExec_t gexec[2] = {nullptr, nullptr};  // by the buffer set that is current when a block starts
   int* d_it = nullptr;
   int dev_it = -1;
   // persistent whole-step kernel (small grids): CTAs and threads per CTA of
@@ -272,6 +272,6 @@ unsigned long long bc_take_adjoint();
 // CUDA graph of one DFT block of steps.
 bool graph_ready(const iris_engine* E, int it, int left);
 void graph_reset(iris_engine* E);
-int graph_block(iris_engine* E, int it, const std::function<void()>& record);
+int graph_block(iris_engine* E, int it, int set, const std::function<void()>& record);
 
 }  // namespace iris
